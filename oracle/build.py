@@ -32,7 +32,7 @@ def build_all(force=False):
     sys.path.insert(0, HERE)
     import build_ref
     ref = build_ref.default_reference_root()
-    if os.path.isdir(ref):
+    if all(os.path.exists(os.path.join(ref, s)) for s in build_ref.SOURCES):
         out.append(build_ref.build(ref, force))
     elif os.path.exists(build_ref.LIB):
         out.append(build_ref.LIB)
