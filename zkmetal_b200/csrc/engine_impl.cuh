@@ -243,7 +243,9 @@ void Engine::enqueue_reduce(const Plan& pl, const void* bucket_base, uint32_t* d
         rc ^= 1;
     }
     if (ev) prof_mark(*ev, 4);
-    k_combine<C><<<nd, 32 * COMBINE_WARPS, 0, stream>>>(inS, inW, dd, nd, d_results);
+    uint32_t most = 1;
+    for (const auto& d : pl.descs) most = std::max(most, d.nred);
+    k_combine<C><<<nd, combine_threads(most), 0, stream>>>(inS, inW, dd, nd, d_results);
     launches++;
     ZK_CUDA(cudaGetLastError());
     if (ev) prof_mark(*ev, 5);

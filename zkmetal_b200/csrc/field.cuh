@@ -346,41 +346,6 @@ ZK_DEV void fe_from_mont(Fe<P>& r, const Fe<P>& a) {
     fe_reduce_once(r, x);
 }
 
-// ------------------------------------------------------------ inversion
-// Binary extended Euclid on integers (Guide to ECC, Hankerson-Menezes-
-// Vanstone, Algorithm 2.22) applied to the Montgomery representative:
-// with a = x*R, it returns (a^-1 mod p) then multiplies by R^3 via two
-// Montgomery products with R2, giving x^-1 * R.  Not constant time (inputs
-// are public).  Zero maps to zero.
-
-template <class P>
-ZK_DEV bool fe_is_one_int(const Fe<P>& a) {
-    uint32_t t = a.v[0] ^ 1u;
-#pragma unroll
-    for (int i = 1; i < P::N; i++) t |= a.v[i];
-    return t == 0;
-}
-
-template <class P>
-ZK_DEV void fe_half_mod(Fe<P>& x) {
-    // x = x/2 mod p for x < p
-    constexpr int N = P::N;
-    if (x.v[0] & 1) {
-        uint32_t c;
-        asm volatile("add.cc.u32 %0, %0, %1;" : "+r"(x.v[0]) : "r"(P::P(0)));
-#pragma unroll
-        for (int i = 1; i < N; i++) asm volatile("addc.cc.u32 %0, %0, %1;" : "+r"(x.v[i]) : "r"(P::P(i)));
-        asm volatile("addc.u32 %0, 0, 0;" : "=r"(c));
-#pragma unroll
-        for (int i = 0; i < N - 1; i++) x.v[i] = __funnelshift_r(x.v[i], x.v[i + 1], 1);
-        x.v[N - 1] = (x.v[N - 1] >> 1) | (c << 31);
-    } else {
-#pragma unroll
-        for (int i = 0; i < N - 1; i++) x.v[i] = __funnelshift_r(x.v[i], x.v[i + 1], 1);
-        x.v[N - 1] >>= 1;
-    }
-}
-
 template <class P>
 ZK_DEV bool fe_geq_int(const Fe<P>& a, const Fe<P>& b) {
     constexpr int N = P::N;
@@ -401,55 +366,179 @@ ZK_DEV void fe_sub_int(Fe<P>& r, const Fe<P>& a, const Fe<P>& b) {
     asm volatile("subc.u32 %0, %1, %2;" : "=r"(r.v[N - 1]) : "r"(a.v[N - 1]), "r"(b.v[N - 1]));
 }
 
+// ------------------------------------------------------------ inversion
+// Division steps of Bernstein and Yang ("Fast constant-time gcd computation
+// and modular inversion", 2019), delta starting at 1/2 (kept doubled): from
+// f = p, g = a, each step halves g after making it even with f, swapping the
+// roles when delta > 0 and g is odd; f ends as +-gcd when g = 0.  INV_STEPS
+// steps at a time run on the low words alone and give a matrix (u v; q r)
+// with (f, g) <- (u f + v g, q f + r g) / 2^INV_STEPS, applied then to the
+// whole numbers and, mod p, to the cofactors d, e (d*a = f, e*a = g mod p,
+// so d*f = 1/a at the end).  Numbers are signed 30-bit limbs.
+// A chain of dependent instructions either way, but every step is the same
+// short branch-free sequence: all lanes of a warp invert in lockstep, and a
+// lone inversion needs no 12-limb shift or comparison per bit, as a binary
+// Euclid does.  Not constant time (the loop ends when g = 0; inputs are
+// public).  Zero, and anything not invertible, maps to zero.
+
+constexpr int INV_STEPS = 30;
+constexpr uint32_t INV_MASK = (1u << INV_STEPS) - 1;
+
+template <class P>
+struct InvLimbs {
+    // d and e grow by at most p/2 per batch from [0, p): below 32p over the
+    // batches of any input (381 bits: at most 30), plus a sign bit
+    static constexpr int L = (P::BITS + 6 + INV_STEPS - 1) / INV_STEPS;
+    static_assert(30 * L >= 32 * P::N - 2 || P::BITS + 6 <= 30 * L, "limbs hold f, g, d and e");
+    // limb i of k-bit-limb p
+    __host__ __device__ static constexpr uint32_t p(int i) {
+        const int w = 30 * i / 32, s = 30 * i % 32;
+        const uint64_t lo = w < P::N ? P::P(w) : 0u, hi = w + 1 < P::N ? P::P(w + 1) : 0u;
+        return (uint32_t)((lo | hi << 32) >> s) & INV_MASK;
+    }
+};
+
+// 32-bit limbs -> 30-bit limbs (the value is below 2^(30 L - 1))
+template <class P>
+ZK_DEV void inv_split(int32_t (&x)[InvLimbs<P>::L], const Fe<P>& a) {
+#pragma unroll
+    for (int i = 0; i < InvLimbs<P>::L; i++) {
+        const int w = 30 * i / 32, s = 30 * i % 32;
+        const uint32_t lo = w < P::N ? a.v[w] : 0u, hi = w + 1 < P::N ? a.v[w + 1] : 0u;
+        x[i] = (int32_t)(__funnelshift_r(lo, hi, s) & INV_MASK);
+    }
+}
+
 template <class P>
 __device__ __noinline__ void fe_inv(Fe<P>& r, const Fe<P>& a) {
-    if (fe_is_zero(a)) {
+    using IL = InvLimbs<P>;
+    constexpr int L = IL::L;
+    int32_t f[L], g[L], d[L], e[L];
+    Fe<P> t;
+#pragma unroll
+    for (int i = 0; i < P::N; i++) t.v[i] = P::R2(i);
+    inv_split<P>(g, a);
+    inv_split<P>(e, t);  // e starts at R^2: (xR)^-1 * R^2 = x^-1 * R
+#pragma unroll
+    for (int i = 0; i < L; i++) {
+        f[i] = (int32_t)IL::p(i);
+        d[i] = 0;
+    }
+    int32_t delta = 1;  // twice delta
+    // 2 * BITS + 64 steps are more than enough for any input (the proven
+    // bound is about 2.3 per bit); the cap only bounds the loop
+#pragma unroll 1
+    for (int batch = 0; batch < (3 * P::BITS + 64) / INV_STEPS; batch++) {
+        uint32_t nz = 0;
+#pragma unroll
+        for (int i = 0; i < L; i++) nz |= (uint32_t)g[i];
+        if (nz == 0) break;
+        int32_t u = 1, v = 0, q = 0, w = 1;
+        uint32_t fl = (uint32_t)f[0] | (uint32_t)f[1] << 30, gl = (uint32_t)g[0] | (uint32_t)g[1] << 30;
+#pragma unroll 10
+        for (int k = 0; k < INV_STEPS; k++) {
+            const bool odd = gl & 1u, swap = odd && delta > 0;
+            // what an odd g takes: f, or -f when the roles swap
+            const uint32_t fa = swap ? 0u - fl : fl;
+            const int32_t ua = swap ? -u : u, va = swap ? -v : v;
+            fl = swap ? gl : fl;
+            u = swap ? q : u;
+            v = swap ? w : v;
+            gl = (gl + (odd ? fa : 0u)) >> 1;
+            q += odd ? ua : 0;
+            w += odd ? va : 0;
+            u <<= 1;
+            v <<= 1;
+            delta = (swap ? -delta : delta) + 2;
+        }
+        // apply the matrix; the low INV_STEPS bits of each f, g sum are zero,
+        // and a multiple m*p (|m| <= 2^29) clears those of d and e
+        int64_t cf = (int64_t)u * f[0] + (int64_t)v * g[0], cg = (int64_t)q * f[0] + (int64_t)w * g[0];
+        int64_t cd = (int64_t)u * d[0] + (int64_t)v * e[0], ce = (int64_t)q * d[0] + (int64_t)w * e[0];
+        // sign-extended low 30 bits of sum * (-1/p)
+        const int32_t md = (int32_t)(((uint32_t)cd * P::N0R()) << 2) >> 2;
+        const int32_t me = (int32_t)(((uint32_t)ce * P::N0R()) << 2) >> 2;
+        cd += (int64_t)md * IL::p(0);
+        ce += (int64_t)me * IL::p(0);
+        cf >>= INV_STEPS;
+        cg >>= INV_STEPS;
+        cd >>= INV_STEPS;
+        ce >>= INV_STEPS;
+#pragma unroll
+        for (int i = 1; i < L; i++) {
+            cf += (int64_t)u * f[i] + (int64_t)v * g[i];
+            cg += (int64_t)q * f[i] + (int64_t)w * g[i];
+            cd += (int64_t)u * d[i] + (int64_t)v * e[i] + (int64_t)md * IL::p(i);
+            ce += (int64_t)q * d[i] + (int64_t)w * e[i] + (int64_t)me * IL::p(i);
+            f[i - 1] = (int32_t)((uint32_t)cf & INV_MASK);
+            g[i - 1] = (int32_t)((uint32_t)cg & INV_MASK);
+            d[i - 1] = (int32_t)((uint32_t)cd & INV_MASK);
+            e[i - 1] = (int32_t)((uint32_t)ce & INV_MASK);
+            cf >>= INV_STEPS;
+            cg >>= INV_STEPS;
+            cd >>= INV_STEPS;
+            ce >>= INV_STEPS;
+        }
+        f[L - 1] = (int32_t)cf;
+        g[L - 1] = (int32_t)cg;
+        d[L - 1] = (int32_t)cd;
+        e[L - 1] = (int32_t)ce;
+    }
+    // f = +-1 (the limbs of -1 are all-ones with a negative top limb)
+    uint32_t one = (uint32_t)f[0] ^ 1u, mone = (uint32_t)f[0] ^ INV_MASK, left = 0;
+#pragma unroll
+    for (int i = 1; i < L; i++) {
+        one |= (uint32_t)f[i];
+        mone |= (uint32_t)f[i] ^ (i == L - 1 ? 0xffffffffu : INV_MASK);
+    }
+#pragma unroll
+    for (int i = 0; i < L; i++) left |= (uint32_t)g[i];
+    if (left || (one && mone)) {
         fe_set_zero(r);
         return;
     }
-    Fe<P> u = a, v, x1, x2;
+    // |d| < 32p to [0, p]: add or subtract 16p, 8p, .., p against the sign of
+    // d (times f's sign first), then p once more if negative
+    const int32_t sg = one ? -1 : 1;
 #pragma unroll
-    for (int i = 0; i < P::N; i++) v.v[i] = P::P(i);
-    fe_set_zero(x1);
-    x1.v[0] = 1;
-    fe_set_zero(x2);
-    // invariant: x1*a = u, x2*a = v (mod p).  Each pass removes at least one
-    // bit from u*v, so 2*32N passes suffice for a canonical nonzero input;
-    // the caps keep a malformed input (a >= p) from looping forever.
-    int guard = 2 * 32 * P::N + 2;
-    while (!fe_is_one_int(u) && !fe_is_one_int(v) && --guard > 0) {
-        if (fe_is_zero(u) || fe_is_zero(v)) break;
-        while ((u.v[0] & 1) == 0) {
+    for (int i = 0; i < L; i++) d[i] *= sg;
+#pragma unroll 1
+    for (int k = 4; k >= -1; k--) {
+        // the sign of d is its top limb's once the limbs are carried
+        int64_t c = 0;
 #pragma unroll
-            for (int i = 0; i < P::N - 1; i++) u.v[i] = __funnelshift_r(u.v[i], u.v[i + 1], 1);
-            u.v[P::N - 1] >>= 1;
-            fe_half_mod(x1);
+        for (int i = 0; i < L; i++) {
+            c += d[i];
+            if (i < L - 1) {
+                d[i] = (int32_t)((uint32_t)c & INV_MASK);
+                c >>= INV_STEPS;
+            } else {
+                d[i] = (int32_t)c;
+            }
         }
-        while ((v.v[0] & 1) == 0) {
+        const bool ng = d[L - 1] < 0;
+        const int32_t s = k < 0 ? (ng ? 1 : 0) : ng ? 1 << k : -(1 << k);
+        c = 0;
 #pragma unroll
-            for (int i = 0; i < P::N - 1; i++) v.v[i] = __funnelshift_r(v.v[i], v.v[i + 1], 1);
-            v.v[P::N - 1] >>= 1;
-            fe_half_mod(x2);
-        }
-        if (fe_geq_int(u, v)) {
-            fe_sub_int(u, u, v);
-            fe_sub(x1, x1, x2);
-        } else {
-            fe_sub_int(v, v, u);
-            fe_sub(x2, x2, x1);
+        for (int i = 0; i < L; i++) {
+            c += d[i] + (int64_t)s * IL::p(i);
+            if (i < L - 1) {
+                d[i] = (int32_t)((uint32_t)c & INV_MASK);
+                c >>= INV_STEPS;
+            } else {
+                d[i] = (int32_t)c;
+            }
         }
     }
-    if (!fe_is_one_int(u) && !fe_is_one_int(v)) {  // not invertible: report zero
-        fe_set_zero(r);
-        return;
-    }
-    Fe<P> ai = fe_is_one_int(u) ? x1 : x2;  // (xR)^-1 as an integer
-    // (xR)^-1 * R2 / R = x^-1 ; again * R2 / R = x^-1 R
-    Fe<P> r2;
 #pragma unroll
-    for (int i = 0; i < P::N; i++) r2.v[i] = P::R2(i);
-    fe_mul(ai, ai, r2);
-    fe_mul(r, ai, r2);
+    for (int i = 0; i < P::N; i++) {
+        const int w0 = 32 * i / 30, s = 32 * i % 30;  // bit 32i lies in limb w0 at s
+        uint64_t x = (uint64_t)(uint32_t)d[w0] >> s;
+        if (w0 + 1 < L) x |= (uint64_t)(uint32_t)d[w0 + 1] << (30 - s);
+        if (w0 + 2 < L && 60 - s < 32) x |= (uint64_t)(uint32_t)d[w0 + 2] << (60 - s);
+        t.v[i] = (uint32_t)x;
+    }
+    fe_reduce_once(r, t);
 }
 
 }  // namespace zkmsm

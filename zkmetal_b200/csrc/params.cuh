@@ -52,6 +52,9 @@ struct Bn254Gen {
     __host__ __device__ static constexpr uint32_t X_MONT(int i) { return (i == 0 ? 0xc58f0d9du : (i == 1 ? 0xd35d438du : (i == 2 ? 0xf5c70b3du : (i == 3 ? 0x0a78eb28u : (i == 4 ? 0x7879462cu : (i == 5 ? 0x666ea36fu : (i == 6 ? 0x9a07df2fu : (i == 7 ? 0x0e0a77c1u : 0u)))))))); }
     __host__ __device__ static constexpr uint32_t Y_MONT(int i) { return (i == 0 ? 0x8b1e1b3au : (i == 1 ? 0xa6ba871bu : (i == 2 ? 0xeb8e167bu : (i == 3 ? 0x14f1d651u : (i == 4 ? 0xf0f28c58u : (i == 5 ? 0xccdd46deu : (i == 6 ? 0x340fbe5eu : (i == 7 ? 0x1c14ef83u : 0u)))))))); }
     static constexpr uint32_t B = 3u;
+    // DBL_C^2 = 3b (DBL_NEG 0) or -3b (DBL_NEG 1): projective doubling chains
+    static constexpr int DBL_NEG = 0;
+    __host__ __device__ static constexpr uint32_t DBL_C_MONT(int i) { return (i == 0 ? 0x50ad28d7u : (i == 1 ? 0x7a17caa9u : (i == 2 ? 0xe15521b9u : (i == 3 ? 0x1f6ac17au : (i == 4 ? 0x696bd284u : (i == 5 ? 0x334bea4eu : (i == 6 ? 0xce179d8eu : (i == 7 ? 0x2a1f6744u : 0u)))))))); }
 };
 
 struct Bls381Fp {
@@ -101,6 +104,9 @@ struct Bls381Gen {
     __host__ __device__ static constexpr uint32_t X_MONT(int i) { return (i == 0 ? 0xfd530c16u : (i == 1 ? 0x5cb38790u : (i == 2 ? 0x9976fff5u : (i == 3 ? 0x7817fc67u : (i == 4 ? 0x143ba1c1u : (i == 5 ? 0x154f95c7u : (i == 6 ? 0xf3d0e747u : (i == 7 ? 0xf0ae6acdu : (i == 8 ? 0x21dbf440u : (i == 9 ? 0xedce6eccu : (i == 10 ? 0x9e0bfb75u : (i == 11 ? 0x12017741u : 0u)))))))))))); }
     __host__ __device__ static constexpr uint32_t Y_MONT(int i) { return (i == 0 ? 0x0ce72271u : (i == 1 ? 0xbaac93d5u : (i == 2 ? 0x7918fd8eu : (i == 3 ? 0x8c22631au : (i == 4 ? 0x570725ceu : (i == 5 ? 0xdd595f13u : (i == 6 ? 0x50405194u : (i == 7 ? 0x51ac5829u : (i == 8 ? 0xad0059c0u : (i == 9 ? 0x0e1c8c3fu : (i == 10 ? 0x5008a26au : (i == 11 ? 0x0bbc3efcu : 0u)))))))))))); }
     static constexpr uint32_t B = 4u;
+    // DBL_C^2 = 3b (DBL_NEG 0) or -3b (DBL_NEG 1): projective doubling chains
+    static constexpr int DBL_NEG = 1;
+    __host__ __device__ static constexpr uint32_t DBL_C_MONT(int i) { return (i == 0 ? 0xe6303e44u : (i == 1 ? 0x3bd8d86du : (i == 2 ? 0x20a968aeu : (i == 3 ? 0x697376c8u : (i == 4 ? 0xd282a50du : (i == 5 ? 0x4ad2b457u : (i == 6 ? 0xcd8e9378u : (i == 7 ? 0x3056d97eu : (i == 8 ? 0x3fd6f0e7u : (i == 9 ? 0xfab1c35cu : (i == 10 ? 0x126f8172u : (i == 11 ? 0x0c592c60u : 0u)))))))))))); }
 };
 
 #ifdef __CUDACC__
@@ -155,6 +161,9 @@ struct Bls377Gen {
     __host__ __device__ static constexpr uint32_t X_MONT(int i) { return (i == 0 ? 0x772451f4u : (i == 1 ? 0x260f33b9u : (i == 2 ? 0x169d5658u : (i == 3 ? 0xc54dd773u : (i == 4 ? 0x69a510ddu : (i == 5 ? 0x5c1551c4u : (i == 6 ? 0x425e1698u : (i == 7 ? 0x761662e4u : (i == 8 ? 0x6f065272u : (i == 9 ? 0xc97d78ccu : (i == 10 ? 0xb361fd4du : (i == 11 ? 0x00a41206u : 0u)))))))))))); }
     __host__ __device__ static constexpr uint32_t Y_MONT(int i) { return (i == 0 ? 0xb8cb81f3u : (i == 1 ? 0x8193961fu : (i == 2 ? 0x5f44adb8u : (i == 3 ? 0x00638d4cu : (i == 4 ? 0xd4daf54au : (i == 5 ? 0xfafaf3dau : (i == 6 ? 0xd655cd18u : (i == 7 ? 0xc27849e2u : (i == 8 ? 0x01d52814u : (i == 9 ? 0x2ec3ddb4u : (i == 10 ? 0x26303c71u : (i == 11 ? 0x007da933u : 0u)))))))))))); }
     static constexpr uint32_t B = 1u;
+    // DBL_C^2 = 3b (DBL_NEG 0) or -3b (DBL_NEG 1): projective doubling chains
+    static constexpr int DBL_NEG = 0;
+    __host__ __device__ static constexpr uint32_t DBL_C_MONT(int i) { return (i == 0 ? 0x8894e1e4u : (i == 1 ? 0x3fabdfd0u : (i == 2 ? 0xcc1f55aau : (i == 3 ? 0xcbf921ddu : (i == 4 ? 0x460edc0cu : (i == 5 ? 0xd17deff1u : (i == 6 ? 0x7897028du : (i == 7 ? 0xd394e81eu : (i == 8 ? 0x0912681au : (i == 9 ? 0xc29c995du : (i == 10 ? 0xaff9d568u : (i == 11 ? 0x01515e6cu : 0u)))))))))))); }
 };
 
 // BN254 G2: GLV with psi(x, y) = (conj(x) * GAMMA1, conj(y) * GAMMA2) = LAMBDA * (x, y)

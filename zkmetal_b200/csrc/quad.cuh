@@ -1,0 +1,236 @@
+// Point arithmetic by quads: four neighbouring lanes hold one XYZZ point, one
+// coordinate each (lane 0: X, 1: Y, 2: ZZ, 3: ZZZ), and share its products.
+//
+// Bound.  A Montgomery product occupies a lone warp's scheduler for ~830
+// cycles at 8 limbs (560 of them heavy-pipe issue), so a chain of XYZZ
+// additions in one thread (14 products, at most two overlapping) costs 8.7 us
+// per addition on a B200 however few points are in flight.  The products of
+// an addition form four layers of at most four independent ones (a doubling:
+// three, and two in the projective form below), so a quad runs an addition in
+// four product times, with the same number of product slots (16 against 14),
+// and a warp keeps eight points.  Values pass between lanes by shuffles.
+// Used where points are few and the chain of additions is the time; kernels
+// with enough points to fill the multiply pipe keep one point per thread.
+//
+// Every lane of the warp calls these functions together (full-mask shuffles;
+// branches are warp-uniform); a lane without work holds the identity (0).
+#pragma once
+#include "types.cuh"
+
+namespace zkmsm {
+
+// the value of quad lane `src` (may differ per lane)
+template <class P>
+ZK_DEV void quad_get(Fe<P>& r, const Fe<P>& a, uint32_t src) {
+#pragma unroll
+    for (int i = 0; i < P::N; i++) r.v[i] = __shfl_sync(0xffffffffu, a.v[i], src, 4);
+}
+
+// the value of the lane two further (X <-> ZZ, Y <-> ZZZ)
+template <class P>
+ZK_DEV void quad_swap2(Fe<P>& r, const Fe<P>& a) {
+#pragma unroll
+    for (int i = 0; i < P::N; i++) r.v[i] = __shfl_xor_sync(0xffffffffu, a.v[i], 2);
+}
+
+template <class P>
+ZK_DEV void fe_select(Fe<P>& r, bool c, const Fe<P>& x, const Fe<P>& y) {
+#pragma unroll
+    for (int i = 0; i < P::N; i++) r.v[i] = c ? x.v[i] : y.v[i];
+}
+
+// quad lane `src`'s flag
+ZK_DEV bool quad_flag(bool f, uint32_t src) { return __shfl_sync(0xffffffffu, f ? 1u : 0u, src, 4) != 0; }
+
+// coordinate q of src[...] (16-byte loads)
+template <class P>
+ZK_DEV void quad_load(Fe<P>& a, const Xyzz<P>* __restrict__ src, uint32_t q) {
+    const uint4* s = reinterpret_cast<const uint4*>(src) + q * (P::N / 4);
+#pragma unroll
+    for (int i = 0; i < P::N / 4; i++) {
+        const uint4 v = s[i];
+        a.v[4 * i] = v.x; a.v[4 * i + 1] = v.y; a.v[4 * i + 2] = v.z; a.v[4 * i + 3] = v.w;
+    }
+}
+
+template <class P>
+ZK_DEV void quad_store(Xyzz<P>* dst, const Fe<P>& a, uint32_t q) {
+    uint4* d = reinterpret_cast<uint4*>(dst) + q * (P::N / 4);
+#pragma unroll
+    for (int i = 0; i < P::N / 4; i++)
+        d[i] = make_uint4(a.v[4 * i], a.v[4 * i + 1], a.v[4 * i + 2], a.v[4 * i + 3]);
+}
+
+// a = 2a (dbl-2008-s-1), three layers; the identity and 2-torsion give 0
+template <class P>
+ZK_DEV void quad_dbl(Fe<P>& a, uint32_t q) {
+    const bool z = fe_is_zero(a);
+    // ZZ = 0 or Y = 0 (both flags fetched by every lane: no short circuit
+    // around a shuffle)
+    const bool zz0 = quad_flag(z, 2), y0 = quad_flag(z, 1), zero = zz0 | y0;
+    Fe<P> y, u, m1, v, x, w, m2, m3, t;
+    quad_get(y, a, 1);
+    fe_dbl(u, y);                      // U = 2Y
+    fe_select(x, q == 0, a, u);
+    fe_mul(m1, x, x);                  // X^2 | V = U^2
+    quad_get(v, m1, 1);
+    quad_get(t, m1, 0);
+    fe_dbl(w, t);
+    fe_add(w, w, t);                   // M = 3X^2
+    fe_select(x, q == 1, u, a);
+    fe_select(x, q == 3, w, x);
+    fe_select(t, q == 3, w, v);
+    fe_mul(m2, x, t);                  // S = X*V | W = U*V | ZZ3 = ZZ*V | M^2
+    Fe<P> s, mm, x3;
+    quad_get(s, m2, 0);
+    quad_get(mm, m2, 3);
+    fe_sub(mm, mm, s);
+    fe_sub(x3, mm, s);                 // X3 = M^2 - 2S
+    fe_sub(s, s, x3);
+    quad_get(t, m2, 1);                // W
+    fe_select(x, q == 0, w, a);        // M | Y | - | ZZZ
+    fe_select(t, q == 0, s, t);        // S - X3 | W | - | W
+    fe_mul(m3, x, t);                  // M(S - X3) | W*Y | - | ZZZ3 = W*ZZZ
+    quad_get(t, m3, 0);
+    fe_sub(t, t, m3);                  // Y3, lane 1
+    fe_select(a, q == 1, t, m3);
+    fe_select(a, q == 0, x3, a);
+    fe_select(a, q == 2, m2, a);
+    if (zero) fe_set_zero(a);
+}
+
+// a += b (add-2008-s), four layers; the identity on either side, P + P and
+// P + (-P) handled
+template <class P>
+ZK_DEV void quad_add(Fe<P>& a, const Fe<P>& b, uint32_t q) {
+    const bool hi = q & 2u;
+    const bool ida = quad_flag(fe_is_zero(a), 2), idb = quad_flag(fe_is_zero(b), 2);
+    Fe<P> m1, m2, m3, m4, d, x, y, pp;
+    quad_swap2(x, b);
+    fe_mul(m1, a, x);                  // U1 = X1*ZZ2 | S1 = Y1*ZZZ2 | U2 = ZZ1*X2 | S2 = ZZZ1*Y2
+    quad_swap2(x, m1);
+    fe_select(y, hi, m1, x);
+    fe_select(x, hi, x, m1);
+    fe_sub(d, y, x);                   // P = U2 - U1 | R = S2 - S1 | P | R
+    const bool zd = fe_is_zero(d);
+    const bool p0 = quad_flag(zd, 0), r0 = quad_flag(zd, 1);
+    fe_select(x, hi, a, d);
+    fe_select(y, hi, b, d);
+    fe_mul(m2, x, y);                  // PP | R^2 | ZZ1*ZZ2 | ZZZ1*ZZZ2
+    quad_get(pp, m2, 0);
+    quad_get(x, d, 0);
+    fe_select(y, q == 0, m1, m2);
+    fe_select(x, q & 1u, x, y);
+    fe_mul(m3, x, pp);                 // Q = U1*PP | PPP = P*PP | ZZ3 | PPP
+    Fe<P> x3, qq, r;
+    quad_get(x3, m2, 1);
+    quad_get(x, m3, 1);
+    quad_get(qq, m3, 0);
+    fe_sub(x3, x3, x);
+    fe_sub(x3, x3, qq);
+    fe_sub(x3, x3, qq);                // X3 = R^2 - PPP - 2Q
+    fe_sub(qq, qq, x3);
+    quad_get(r, d, 1);
+    fe_select(x, q == 1, m1, m2);
+    fe_select(x, q == 0, r, x);
+    fe_select(y, q == 0, qq, m3);
+    fe_mul(m4, x, y);                  // R(Q - X3) | S1*PPP | - | ZZZ3 = ZZZ1*ZZZ2*PPP
+    quad_get(x, m4, 0);
+    fe_sub(x, x, m4);                  // Y3, lane 1
+    fe_select(y, q == 0, x3, m4);
+    fe_select(y, q == 1, x, y);
+    fe_select(y, q == 2, m3, y);
+    const bool same = !ida && !idb && p0 && r0;
+    if (__any_sync(0xffffffffu, same)) {  // P + P (rare): the whole warp doubles
+        x = a;
+        quad_dbl(x, q);
+        fe_select(y, same, x, y);
+    }
+    if (!same && p0 && !ida && !idb) fe_set_zero(y);  // P + (-P)
+    fe_select(y, ida, b, y);
+    fe_select(a, idb, a, y);
+}
+
+// ------------------------------------------------------- chains of doublings
+// 2^count * point for long chains, in homogeneous coordinates: X/Z, Y/Z.  The
+// doubling for a = 0 of Renes, Costello and Batina ("Complete addition
+// formulas for prime order elliptic curves", 2016) is, with B = 3b*Z^2,
+//   X3 = 2XY (Y^2 - 3B),  Y3 = (Y^2 - 3B)(Y^2 + B) + 8 Y^2 B,  Z3 = 8 Y^3 Z:
+// two layers of four products where XYZZ needs three.  B takes no product by
+// b: the chain carries W = c*Z with c^2 = +-3b (DBL_C, DBL_NEG in the curve's
+// parameters), so that B = +-W^2.  Quad lanes: X, Y, W, W.
+template <class C>
+struct QuadChain {
+    using P = typename C::Fp;
+
+    // XYZZ -> (X*ZZZ, Y*ZZ, c*ZZ*ZZZ); the identity becomes all zeros, which
+    // doubling keeps
+    static ZK_DEV void enter(Fe<P>& a, uint32_t q) {
+        Fe<P> t, c;
+        quad_get(t, a, q == 1 ? 2 : 3);
+        quad_get(a, a, q == 3 ? 2 : q);
+        fe_mul(a, a, t);               // X*ZZZ | Y*ZZ | ZZ*ZZZ | ZZ*ZZZ
+#pragma unroll
+        for (int i = 0; i < P::N; i++) c.v[i] = C::Gen::DBL_C_MONT(i);
+        fe_mul(t, a, c);
+        fe_select(a, q & 2u, t, a);
+    }
+
+    static ZK_DEV void dbl(Fe<P>& a, uint32_t q) {
+        Fe<P> y, m1, A, B, t, s, u, v, x;
+        quad_get(y, a, 1);
+        fe_dbl(x, y);
+        fe_select(x, q == 0 || q == 3, x, a);
+        fe_mul_x<true>(m1, a, x);      // 2XY | A = Y^2 | W^2 | 2YW
+        quad_get(A, m1, 1);
+        quad_get(B, m1, 2);
+        fe_dbl(v, B);                  // 2B
+        fe_add(t, v, B);               // 3B
+        if (C::Gen::DBL_NEG) {
+            fe_add(t, A, t);
+            fe_sub(s, A, B);
+        } else {
+            fe_sub(t, A, t);           // Y^2 - 3B
+            fe_add(s, A, B);           // Y^2 + B
+        }
+        fe_dbl(u, A);
+        fe_dbl(u, u);                  // 4Y^2
+        quad_get(x, m1, q == 2 ? 3 : q);
+        fe_select(x, q == 1, t, x);
+        fe_select(x, q == 3, u, x);    // 2XY | t | 2YW | u
+        fe_select(y, q == 1, s, t);
+        fe_select(y, q == 2, u, y);
+        fe_select(y, q == 3, v, y);    // t | s | u | v
+        fe_mul_x<true>(m1, x, y);      // X3 | t*s | W3 | 8 Y^2 |B|
+        quad_get(x, m1, q == 1 ? 3 : 2);
+        if (C::Gen::DBL_NEG) fe_sub(y, m1, x);
+        else fe_add(y, m1, x);
+        fe_select(a, q == 1, y, m1);
+        fe_select(a, q == 3, x, a);
+    }
+
+    // back to XYZZ with ZZ = W^2: x = cX / W = (cX*W) / W^2
+    static ZK_DEV void leave(Fe<P>& a, uint32_t q) {
+        Fe<P> c, t, w, m;
+#pragma unroll
+        for (int i = 0; i < P::N; i++) c.v[i] = C::Gen::DBL_C_MONT(i);
+        fe_select(t, q & 2u, a, c);
+        fe_mul(m, a, t);               // cX | cY | W^2 | W^2
+        quad_get(w, a, 2);
+        quad_get(t, m, 2);
+        fe_select(t, q == 1, t, w);
+        fe_mul(t, m, t);               // cX*W | cY*W^2 | - | W^3
+        fe_select(a, q == 2, m, t);
+    }
+};
+
+// BN254 G2: 3b = 9 / (9 + u) has no cheap form there; the chain stays XYZZ
+template <>
+struct QuadChain<Bn254G2> {
+    using P = Bn254G2::Fp;
+    static ZK_DEV void enter(Fe<P>&, uint32_t) {}
+    static ZK_DEV void dbl(Fe<P>& a, uint32_t q) { quad_dbl(a, q); }
+    static ZK_DEV void leave(Fe<P>&, uint32_t) {}
+};
+
+}  // namespace zkmsm

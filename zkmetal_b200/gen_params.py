@@ -133,6 +133,26 @@ def g2_psi_check(p, r, G, gam1, gam2, lam):
     return on and psi == mul(P, lam)
 
 
+def field_sqrt(a, p):
+    """The smaller square root of a mod p (Tonelli-Shanks)."""
+    a %= p
+    assert pow(a, (p - 1) // 2, p) == 1
+    q, m = p - 1, 0
+    while q % 2 == 0:
+        q, m = q // 2, m + 1
+    z = next(z for z in range(2, 1000) if pow(z, (p - 1) // 2, p) == p - 1)
+    c, t, r = pow(z, q, p), pow(a, q, p), pow(a, (q + 1) // 2, p)
+    while t != 1:
+        i, t2 = 0, t
+        while t2 != 1:
+            i, t2 = i + 1, t2 * t2 % p
+        b = pow(c, 1 << (m - i - 1), p)
+        m, c = i, b * b % p
+        t, r = t * c % p, r * b % p
+    assert r * r % p == a
+    return min(r, p - r)
+
+
 def limbs(x, n):
     return [(x >> (32 * i)) & 0xFFFFFFFF for i in range(n)]
 
@@ -292,6 +312,11 @@ def emit():
         out.append(fn_table("X_MONT", limbs(G[0] * R % p, N)))
         out.append(fn_table("Y_MONT", limbs(G[1] * R % p, N)))
         out.append("    static constexpr uint32_t B = %du;\n" % b)
+        out.append("    // DBL_C^2 = 3b (DBL_NEG 0) or -3b (DBL_NEG 1): projective doubling chains\n")
+        neg = pow(3 * b, (p - 1) // 2, p) != 1
+        c = field_sqrt(-3 * b if neg else 3 * b, p)
+        out.append("    static constexpr int DBL_NEG = %d;\n" % neg)
+        out.append(fn_table("DBL_C_MONT", limbs(c * R % p, N)))
         out.append("};\n\n")
     # BN254 G2 generator (Fp2 coordinates c0 limbs then c1 limbs, Montgomery)
     g2_check(P_BN, R_BN, G2_BN)
