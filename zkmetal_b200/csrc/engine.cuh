@@ -261,7 +261,9 @@ struct Plan {
     // scatter groups of pass 1 and the chunk-count bound of pass 2
     uint32_t msd_passes = 0, msd_bits1 = 0, msd_bits2 = 0, msd_tiles1 = 0, msd_tiles2 = 0;
     uint32_t msd_groups1 = 0, msd_chunks2 = 0;
-    // segmented-sum levels: chunk length and chunk-count bound per level
+    // segmented-sum levels: chunk length and chunk-count bound per level;
+    // acc_fold: the first level runs k_acc_fold too (else k_acc_l1)
+    bool acc_fold = false;
     std::vector<uint32_t> acc_K, acc_T;
     std::vector<uint64_t> acc_Mbound;
     // bucket-reduction levels
@@ -286,6 +288,7 @@ struct Plan {
         red_L = 8;
         red_log2L = 3;
         acc_threads = 0;
+        acc_fold = false;
         acc_K.clear();
         acc_T.clear();
         acc_Mbound.clear();
@@ -584,9 +587,9 @@ class Engine {
     }
 
     // workspace
-    DevBuf w_points, w_phi, w_scalars, w_counts, w_offsets, w_cursor, w_ents, w_buckets;
+    DevBuf w_points, w_phi, w_scalars, w_ents, w_buckets;
     DevBuf w_ents2, w_thist, w_stripe_buckets, w_seg;
-    DevBuf w_cnt, w_pos, w_tiles, w_totals, w_pkeys[2], w_pvals[2], w_redS[2], w_redW[2];
+    DevBuf w_tiles, w_totals, w_pkeys[2], w_pvals[2], w_redS[2], w_redW[2];
     DevBuf w_results, w_comb, w_profile;
     uint32_t* h_profile = nullptr;  // pinned, PROFILE_BINS words
     bool comb_ready[NCURVES] = {};
@@ -597,8 +600,8 @@ class Engine {
     // memory pool keeps at least 4 GiB of freed blocks for reuse (a larger
     // setting, e.g. a server's reservation, is left as it is).
     void bind_workspace_stream() {
-        DevBuf* bufs[] = {&w_points, &w_phi, &w_scalars, &w_counts, &w_offsets, &w_cursor, &w_ents, &w_buckets,
-                          &w_ents2, &w_thist, &w_stripe_buckets, &w_seg, &w_cnt, &w_pos, &w_tiles, &w_totals,
+        DevBuf* bufs[] = {&w_points, &w_phi, &w_scalars, &w_ents, &w_buckets,
+                          &w_ents2, &w_thist, &w_stripe_buckets, &w_seg, &w_tiles, &w_totals,
                           &w_pkeys[0], &w_pkeys[1], &w_pvals[0], &w_pvals[1], &w_redS[0], &w_redS[1],
                           &w_redW[0], &w_redW[1], &w_results, &w_comb, &w_profile, &transient.d_descs,
                           &transient.d_tasks};
@@ -852,16 +855,21 @@ class Engine {
             if (sc.chunk_pct > 0)
                 K1 = (uint32_t)std::min<uint64_t>(4096, std::max<uint64_t>(8, (uint64_t)K1 * sc.chunk_pct / 100));
         }
-        uint32_t K = K1;
+        // fold levels: few leaves per quad while a level is latency-bound,
+        // more when its blocks fill the device several times over
+        auto fold_chunk = [](uint64_t m) { return FOLD_QUADS * (m <= (1ull << 18) ? 4u : 16u); };
+        pl.acc_fold = tuning.chunk <= 0 && M <= ACC_FOLD_MAX_ENTRIES;
+        uint32_t K = pl.acc_fold ? fold_chunk(M) : K1;
         for (int lvl = 0; lvl < 40; lvl++) {
             uint64_t T = (M + K - 1) / K;
             if (T == 0) T = 1;
             pl.acc_K.push_back(K);
             pl.acc_T.push_back((uint32_t)T);
             pl.acc_Mbound.push_back(M);
-            if (T <= 1) break;
+            // k_acc_l1 always leaves its boundary runs to a level after it
+            if (T <= 1 && (lvl > 0 || pl.acc_fold)) break;
             M = 2 * T;
-            K = 16;
+            K = fold_chunk(M);
         }
         // reduction levels
         std::vector<RedTask> lvl0;
@@ -979,8 +987,6 @@ class Engine {
         using P = typename C::Fp;
         const size_t xs = sizeof(Xyzz<P>);
         bool grew = false;
-        grew |= w_counts.ensure(((size_t)pl.nbuckets + 1) * 4);
-        grew |= w_cursor.ensure(((size_t)pl.nbuckets + 1) * 4);
         grew |= w_ents.ensure(pl.entry_bound * 8 + 16);
         uint64_t hsz = (uint64_t)(1u << pl.sort_bits) * pl.sort_tiles;
         if (pl.msd_passes) {
@@ -992,11 +998,9 @@ class Engine {
         grew |= w_ents2.ensure(pl.entry_bound * 8 + 16);
         grew |= w_thist.ensure(hwords * 4 + 16);
         grew |= w_buckets.ensure((size_t)pl.nbuckets * xs + xs);
-        uint64_t tmax = 1, m2 = 1, m3 = 1;
-        for (size_t l = 0; l < pl.acc_T.size(); l++) tmax = std::max<uint64_t>(tmax, pl.acc_T[l]);
+        uint64_t m2 = 2, m3 = 2;
         if (pl.acc_Mbound.size() > 1) m2 = pl.acc_Mbound[1];
         for (size_t l = 2; l < pl.acc_Mbound.size(); l++) m3 = std::max<uint64_t>(m3, pl.acc_Mbound[l]);
-        grew |= w_cnt.ensure(tmax * 4 + 16);
         grew |= w_pkeys[0].ensure(m2 * 4 + 16);
         grew |= w_pvals[0].ensure(m2 * xs + xs);
         grew |= w_pkeys[1].ensure(m3 * 4 + 16);
@@ -1012,8 +1016,7 @@ class Engine {
         }
         grew |= w_results.ensure((pl.descs.size() + 1) * 3 * P::N * 4);
         // scan tile sums for the longest scanned array (no allocation inside enqueue)
-        grew |= w_tiles.ensure(((std::max<uint64_t>(std::max<uint64_t>(pl.nbuckets, tmax), hsz) + 2047) / 2048 + 2) *
-                               4);
+        grew |= w_tiles.ensure(((std::max<uint64_t>(pl.nbuckets, hsz) + 2047) / 2048 + 2) * 4);
         if (grew) {
             drop_graphs();  // captured graphs hold the old addresses
             workspace_growths++;

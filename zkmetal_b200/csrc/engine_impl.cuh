@@ -170,41 +170,31 @@ void Engine::enqueue(const Plan& pl, const uint32_t* d_bases, const uint32_t* d_
     }
     prof_mark(ev, 1);
     // segmented sums
-    const uint32_t* keys = w_ents.as<uint32_t>();  // level 1: keys are the .x of packed entries
-    uint32_t kstride = 2;
     int cur = 0;
     for (size_t l = 0; l < pl.acc_K.size(); l++) {
-        uint32_t K = pl.acc_K[l], T = pl.acc_T[l];
+        const uint32_t K = pl.acc_K[l], T = pl.acc_T[l];
+        const bool last = l + 1 == pl.acc_K.size();
         uint32_t* d_len = tot + l;
         uint32_t* d_next = tot + l + 1;
-        k_chunk_count<<<(T + 255) / 256, 256, 0, stream>>>(keys, kstride, d_len, K, T, w_cnt.as<uint32_t>());
-        launches++;
-        ZK_CUDA(cudaGetLastError());
-        scan_u32(*this, w_cnt.as<uint32_t>(), T, d_next, nullptr);
         uint32_t* okeys = w_pkeys[cur].as<uint32_t>();
         Xyzz<P>* ovals = w_pvals[cur].as<Xyzz<P>>();
-        if (l == 0) {
+        if (l == 0 && !pl.acc_fold) {
             const uint32_t AT = pl.acc_threads && pl.acc_threads <= (uint32_t)AccLaunch<C>::THREADS
                                         ? pl.acc_threads
                                         : (uint32_t)AccLaunch<C>::THREADS;
-            k_acc_l1<C><<<(T + AT - 1) / AT, AT, 0, stream>>>(
-                    w_ents.as<uint2>(), d_len, K, d_bases,
-                                                             d_phi, w_cnt.as<uint32_t>(),
+            k_acc_l1<C><<<(T + AT - 1) / AT, AT, 0, stream>>>(w_ents.as<uint2>(), d_len, K, d_bases, d_phi, d_next,
                                                              buckets, okeys, ovals);
-            launches++;
+        } else if (l == 0) {
+            k_acc_fold<C, true><<<T, FOLD_THREADS, 0, stream>>>(w_ents.as<uint2>(), d_bases, d_phi, nullptr, nullptr,
+                                                                d_len, K / FOLD_QUADS, last, d_next, buckets, okeys,
+                                                                ovals);
         } else {
-            const Xyzz<P>* ivals = w_pvals[cur ^ 1].as<Xyzz<P>>();
-            if (T <= RED_INLINE_MAX_NODES)  // few threads: latency-bound
-                k_acc_lj<C, true><<<(T + 255) / 256, 256, 0, stream>>>(keys, ivals, d_len, K, w_cnt.as<uint32_t>(),
-                                                                       buckets, okeys, ovals);
-            else
-                k_acc_lj<C, false><<<(T + 255) / 256, 256, 0, stream>>>(keys, ivals, d_len, K,
-                                                                        w_cnt.as<uint32_t>(), buckets, okeys, ovals);
-            launches++;
+            k_acc_fold<C, false><<<T, FOLD_THREADS, 0, stream>>>(
+                    nullptr, nullptr, nullptr, w_pkeys[cur ^ 1].as<uint32_t>(), w_pvals[cur ^ 1].as<Xyzz<P>>(), d_len,
+                    K / FOLD_QUADS, last, d_next, buckets, okeys, ovals);
         }
+        launches++;
         ZK_CUDA(cudaGetLastError());
-        keys = okeys;
-        kstride = 1;
         cur ^= 1;
         if (l == 0) prof_mark(ev, 2);
     }

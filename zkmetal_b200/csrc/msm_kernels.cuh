@@ -17,12 +17,14 @@
 //     with global atomics, kept for the allocation-free entry point.)
 //  4. k_acc_l1        bucket accumulation: each thread sums a fixed-length
 //                     chunk of the sorted list with mixed XYZZ additions;
-//                     runs wholly inside a chunk are final buckets, runs cut
-//                     by a chunk edge become partial sums.
+//                     runs strictly inside a chunk are final buckets, a
+//                     chunk's first and last run become partial sums.
 //                     [msm_kernels.metal:16-62]
-//  5. k_acc_lj        the same segmented reduction over the partial sums,
-//                     repeated until no bucket is cut (handles any skew, e.g.
-//                     20% of all points in one bucket for witness scalars).
+//  5. k_acc_fold      the same segmented reduction over the partial sums (in
+//                     small calls over the entries too), quads of lanes and a
+//                     tree per block, repeated until one block is left
+//                     (handles any skew, e.g. 20% of all points in one bucket
+//                     for witness scalars).
 //  6. k_reduce_level  per window sum_b b*B_b by a tree of running sums.
 //                     [msm_kernels.metal:152-248]
 //  7. k_combine       sum of the windows shifted to their bit offsets (a
@@ -877,26 +879,17 @@ __global__ void __launch_bounds__(128) k_shift_affine(const Xyzz<typename C::Fp>
 
 // ------------------------------------------------------------ segmented sums
 
-// Partial-slot count of a chunk: a run touching the chunk's first entry that
-// began earlier, and a run touching its last entry that goes on after it,
-// are partial; a single run that is cut on either side is one partial.
-static __global__ void __launch_bounds__(256) k_chunk_count(const uint32_t* __restrict__ keys, uint32_t kstride,
-                                                     const uint32_t* __restrict__ d_len, uint32_t K,
-                                                     uint32_t nchunks, uint32_t* __restrict__ cnt) {
-    uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nchunks) return;
-    uint32_t M = *d_len;
-    uint64_t start = (uint64_t)t * K;
-    if (start >= M) {
-        cnt[t] = 0;
-        return;
-    }
-    uint32_t end = (uint32_t)(start + K < (uint64_t)M ? start + K : (uint64_t)M);
-    uint32_t k0 = keys[start * kstride], k1 = keys[(uint64_t)(end - 1) * kstride];
-    uint32_t cb = start > 0 && keys[(start - 1) * kstride] == k0;
-    uint32_t ca = end < M && keys[(uint64_t)end * kstride] == k1;
-    cnt[t] = (k0 == k1) ? (cb | ca) : (cb + ca);
-}
+// Bucket sums are segmented sums of the sorted entry list, in levels.  A level
+// cuts its list into chunks; runs of one key strictly inside a chunk are
+// final and go to their buckets, and chunk t hands its first run to slot 2t
+// and its last run to slot 2t + 1 of the next level's list (ACC_EMPTY there
+// when one run fills the chunk), still sorted by key.  Whether a boundary run
+// really goes on in the neighbouring chunk is left to the next level, so no
+// level counts or scans slots (two to four launches a level, which were a
+// third of a small call's launches), and the list length
+// 2 * ceil(length / chunk) needs no host.  The last level is one block, whose
+// boundary runs are final too.
+constexpr uint32_t ACC_EMPTY = 0xffffffffu;  // above every bucket id
 
 // Level 1: chunks of the sorted entry list, mixed additions of gathered bases.
 // Launch shape of k_acc_l1 per curve: BN254 fits two 256-thread blocks per
@@ -920,21 +913,20 @@ __global__ void __launch_bounds__(AccLaunch<C>::THREADS, AccLaunch<C>::MIN_BLOCK
                                                 const uint32_t* __restrict__ d_len, uint32_t K,
                                                 const uint32_t* __restrict__ bases,
                                                 const uint32_t* __restrict__ phi,
-                                                const uint32_t* __restrict__ slot_pos,
+                                                uint32_t* __restrict__ d_next,
                                                 Xyzz<typename C::Fp>* __restrict__ buckets,
                                                 uint32_t* __restrict__ pkeys,
                                                 Xyzz<typename C::Fp>* __restrict__ pvals) {
     using P = typename C::Fp;
     uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t M = *d_len;
+    if (t == 0) *d_next = (uint32_t)(2 * (((uint64_t)M + K - 1) / K));
     uint64_t start64 = (uint64_t)t * K;
     if (start64 >= M) return;
     uint32_t start = (uint32_t)start64;
     uint32_t end = (uint32_t)(start64 + K < (uint64_t)M ? start64 + K : (uint64_t)M);
     uint32_t cur = ents[start].x;
-    bool cont_before = start > 0 && ents[start - 1].x == cur;
     bool first_run = true;
-    uint32_t slot = slot_pos[t];
     Xyzz<P> acc;
     xyzz_set_id(acc);
 #pragma unroll 1
@@ -942,13 +934,8 @@ __global__ void __launch_bounds__(AccLaunch<C>::THREADS, AccLaunch<C>::MIN_BLOCK
         const uint2 e = ents[i];
         const uint32_t k = e.x;
         if (k != cur) {
-            if (first_run && cont_before) {
-                pkeys[slot] = cur;
-                store_xyzz(pvals + slot, acc);
-                slot++;
-            } else {
-                store_xyzz(buckets + cur, acc);
-            }
+            if (first_run) pkeys[2 * t] = cur;
+            store_xyzz(first_run ? pvals + 2 * t : buckets + cur, acc);
             xyzz_set_id(acc);
             cur = k;
             first_run = false;
@@ -961,13 +948,10 @@ __global__ void __launch_bounds__(AccLaunch<C>::THREADS, AccLaunch<C>::MIN_BLOCK
             xyzz_add_affine(acc, q);
         }
     }
-    bool cont_after = end < M && ents[end].x == cur;
-    if ((first_run && cont_before) || cont_after) {
-        pkeys[slot] = cur;
-        store_xyzz(pvals + slot, acc);
-    } else {
-        store_xyzz(buckets + cur, acc);
-    }
+    const uint32_t slot = 2 * t + (first_run ? 0 : 1);
+    pkeys[slot] = cur;
+    store_xyzz(pvals + slot, acc);
+    if (first_run) pkeys[2 * t + 1] = ACC_EMPTY;
 }
 
 // Stripes of one MSM (same window layout, S bucket arrays of nb buckets one
@@ -989,55 +973,170 @@ __global__ void __launch_bounds__(128) k_bucket_fold(Xyzz<typename C::Fp>* __res
     store_xyzz(b + i, acc);
 }
 
-// Level >= 2: the same over partial sums (XYZZ + XYZZ additions).  INL:
-// inline products, for levels of few threads (latency-bound: an inline
-// addition has ~40% less latency than one with out-of-line products).
-template <class C, bool INL>
-__global__ void __launch_bounds__(256) k_acc_lj(const uint32_t* __restrict__ keys,
-                                                const Xyzz<typename C::Fp>* __restrict__ vals,
-                                                const uint32_t* __restrict__ d_len, uint32_t K,
-                                                const uint32_t* __restrict__ slot_pos,
-                                                Xyzz<typename C::Fp>* __restrict__ buckets,
-                                                uint32_t* __restrict__ pkeys,
-                                                Xyzz<typename C::Fp>* __restrict__ pvals) {
-    using P = typename C::Fp;
-    uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t M = *d_len;
-    uint64_t start64 = (uint64_t)t * K;
-    if (start64 >= M) return;
-    uint32_t start = (uint32_t)start64;
-    uint32_t end = (uint32_t)(start64 + K < (uint64_t)M ? start64 + K : (uint64_t)M);
-    uint32_t cur = keys[start];
-    bool cont_before = start > 0 && keys[start - 1] == cur;
-    bool first_run = true;
-    uint32_t slot = slot_pos[t];
-    Xyzz<P> acc;
-    xyzz_set_id(acc);
-#pragma unroll 1
-    for (uint32_t i = start; i < end; i++) {
-        uint32_t k = keys[i];
-        if (k != cur) {
-            if (first_run && cont_before) {
-                pkeys[slot] = cur;
-                store_xyzz(pvals + slot, acc);
-                slot++;
-            } else {
-                store_xyzz(buckets + cur, acc);
-            }
-            xyzz_set_id(acc);
-            cur = k;
-            first_run = false;
-        }
-        Xyzz<P> q;
-        load_xyzz(q, vals + i);
-        xyzz_add<P, INL>(acc, q);
+// The levels after the first, and for small calls the first as well: one
+// block folds FOLD_QUADS * J leaves.  A leaf is one run: a slot of the previous
+// level's list or (ENTS) a sorted entry's point.  Quad i adds up leaves
+// [i*J, (i+1)*J) one after another, then the quads' nodes merge in a tree,
+// three levels inside each warp and three over the eight warps.  A node is
+// the first and last run of its range (one run when `whole`); everything
+// between is final and already in its bucket, so a merge is one addition at
+// most (the left node's last run and the right node's first, when the keys
+// agree).
+//
+// Latency-bound in small calls: J + 5 additions deep per level of 64 J leaves.
+// BN254 at 2^8 points (16k entries, J = 4): two levels, 33 + 20 us, against
+// 57 us for chunks of eight in one thread each, then four levels of sixteen
+// (201 us) with a count and a scan each (21 us).  2^16 points, after
+// k_acc_l1: 179 against 354 us + 45 us of counts and scans.
+template <class P>
+struct FoldNode {
+    Fe<P> l, r;       // this lane's coordinate of the first / last run's sum
+    uint32_t kl, kr;  // their keys; kl = ACC_EMPTY: nothing in the range
+    bool whole;       // the range is one run: l, kl (r, kr unused)
+};
+
+// a = a ++ b for the quads with `on` set (all lanes call)
+template <class P>
+ZK_DEV void fold_merge(FoldNode<P>& a, const FoldNode<P>& b, bool on, uint32_t q, Xyzz<P>* __restrict__ buckets) {
+    on = on && b.kl != ACC_EMPTY;
+    const bool take = on && a.kl == ACC_EMPTY;  // nothing on the left yet
+    const uint32_t ka = a.whole ? a.kl : a.kr;
+    const bool same = on && ka == b.kl;
+    Fe<P> s, x;
+    fe_select(s, a.whole, a.l, a.r);
+    if (__any_sync(0xffffffffu, same)) {
+        fe_set_zero(x);
+        fe_select(x, same, b.l, x);
+        quad_add(s, x, q);
     }
-    bool cont_after = end < M && keys[end] == cur;
-    if ((first_run && cont_before) || cont_after) {
-        pkeys[slot] = cur;
-        store_xyzz(pvals + slot, acc);
+    if (!on) return;
+    if (take) {
+        a = b;
+        return;
+    }
+    // runs that end inside the merged range
+    if (!a.whole && !(same && b.whole)) quad_store(buckets + ka, s, q);
+    if (!same && !b.whole) quad_store(buckets + b.kl, b.l, q);
+    if (same && a.whole) a.l = s;
+    if (same && b.whole) {
+        if (!a.whole) a.r = s;
     } else {
-        store_xyzz(buckets + cur, acc);
+        a.r = b.whole ? b.l : b.r;
+        a.kr = b.whole ? b.kl : b.kr;
+        a.whole = false;
+    }
+}
+
+// the node of the quad `delta` quads further in the warp
+template <class P>
+ZK_DEV void fold_shfl(FoldNode<P>& b, const FoldNode<P>& a, uint32_t delta) {
+#pragma unroll
+    for (int i = 0; i < P::N; i++) {
+        b.l.v[i] = __shfl_down_sync(0xffffffffu, a.l.v[i], 4 * delta);
+        b.r.v[i] = __shfl_down_sync(0xffffffffu, a.r.v[i], 4 * delta);
+    }
+    b.kl = __shfl_down_sync(0xffffffffu, a.kl, 4 * delta);
+    b.kr = __shfl_down_sync(0xffffffffu, a.kr, 4 * delta);
+    b.whole = __shfl_down_sync(0xffffffffu, a.whole ? 1u : 0u, 4 * delta) != 0;
+}
+
+template <class C, bool ENTS>
+__global__ void __launch_bounds__(FOLD_THREADS) k_acc_fold(const uint2* __restrict__ ents,
+                                                           const uint32_t* __restrict__ bases,
+                                                           const uint32_t* __restrict__ phi,
+                                                           const uint32_t* __restrict__ keys,
+                                                           const Xyzz<typename C::Fp>* __restrict__ vals,
+                                                           const uint32_t* __restrict__ d_len, uint32_t J,
+                                                           bool last, uint32_t* __restrict__ d_next,
+                                                           Xyzz<typename C::Fp>* __restrict__ buckets,
+                                                           uint32_t* __restrict__ pkeys,
+                                                           Xyzz<typename C::Fp>* __restrict__ pvals) {
+    using P = typename C::Fp;
+    constexpr uint32_t WARPS = FOLD_THREADS / 32;
+    static_assert(WARPS == 8, "the warps' nodes fill the quads of one warp");
+    __shared__ uint4 sh_raw[WARPS * 2 * sizeof(Xyzz<P>) / sizeof(uint4)];
+    __shared__ uint32_t shk[WARPS], shr[WARPS];
+    __shared__ bool shw[WARPS];
+    Xyzz<P>* sh = reinterpret_cast<Xyzz<P>*>(sh_raw);
+    const uint32_t q = threadIdx.x & 3, quad = threadIdx.x >> 2, warp = threadIdx.x >> 5;
+    const uint32_t M = *d_len, K = FOLD_QUADS * J;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *d_next = (uint32_t)(2 * (((uint64_t)M + K - 1) / K));
+    if ((uint64_t)blockIdx.x * K >= M) return;  // block-uniform
+    const uint64_t i0 = (uint64_t)blockIdx.x * K + (uint64_t)quad * J;
+    FoldNode<P> a, b;
+    fe_set_zero(a.l);
+    a.r = b.r = a.l;
+    a.kl = a.kr = b.kr = ACC_EMPTY;
+    a.whole = true;
+#pragma unroll 1
+    for (uint32_t j = 0; j < J; j++) {
+        const uint64_t i = i0 + j;
+        b.kl = ACC_EMPTY;
+        b.whole = true;
+        fe_set_zero(b.l);
+        if (i < M) {
+            if (ENTS) {
+                const uint2 e = ents[i];
+                b.kl = e.x;
+                // lanes 0 and 1 take x and +-y, lanes 2 and 3 one; the
+                // identity (0, 0) stays all zeros
+                const uint4* s = reinterpret_cast<const uint4*>(((e.y >> 30) & 1 ? phi : bases) +
+                                                                (size_t)(e.y & VAL_IDX_MASK) * 2 * P::N);
+                Affine<P> pt;
+                load_fe(pt.x, s);
+                load_fe(pt.y, s + P::N / 4);
+                if (!affine_is_id(pt)) {
+                    if (e.y >> 31) fe_neg(pt.y, pt.y);
+                    Fe<P> one;
+                    fe_set_one(one);
+                    fe_select(b.l, q == 0, pt.x, pt.y);
+                    fe_select(b.l, q & 2u, one, b.l);
+                }
+            } else {
+                b.kl = keys[i];
+                if (b.kl != ACC_EMPTY) quad_load(b.l, vals + i, q);
+            }
+        }
+        fold_merge(a, b, true, q, buckets);
+    }
+#pragma unroll 1
+    for (uint32_t st = 1; st < 8; st <<= 1) {
+        fold_shfl(b, a, st);
+        fold_merge(a, b, !(quad & (2 * st - 1)), q, buckets);
+    }
+    if (!(quad & 7)) {
+        quad_store(sh + 2 * warp, a.l, q);
+        quad_store(sh + 2 * warp + 1, a.r, q);
+        if (q == 0) {
+            shk[warp] = a.kl;
+            shr[warp] = a.kr;
+            shw[warp] = a.whole;
+        }
+    }
+    __syncthreads();
+    if (warp != 0) return;
+    quad_load(a.l, sh + 2 * quad, q);
+    quad_load(a.r, sh + 2 * quad + 1, q);
+    a.kl = shk[quad];
+    a.kr = shr[quad];
+    a.whole = shw[quad];
+#pragma unroll 1
+    for (uint32_t st = 1; st < WARPS; st <<= 1) {
+        fold_shfl(b, a, st);
+        fold_merge(a, b, !(quad & (2 * st - 1)), q, buckets);
+    }
+    if (quad != 0) return;
+    if (last) {
+        quad_store(buckets + a.kl, a.l, q);
+        if (!a.whole) quad_store(buckets + a.kr, a.r, q);
+    } else {
+        const uint64_t o = 2 * (uint64_t)blockIdx.x;
+        quad_store(pvals + o, a.l, q);
+        if (!a.whole) quad_store(pvals + o + 1, a.r, q);
+        if (q == 0) {
+            pkeys[o] = a.kl;
+            pkeys[o + 1] = a.whole ? ACC_EMPTY : a.kr;
+        }
     }
 }
 

@@ -50,14 +50,12 @@ constexpr uint32_t NWIN = (Bn254Glv::HALF_BITS + 1 + CB - 1) / CB;     // 13 sig
 constexpr uint32_t BPW = 1u << (CB - 1);                               // buckets per window
 constexpr uint32_t NB = NWIN * BPW;                                    // 6656 buckets
 constexpr uint64_t E_MAX = 2ull * N_MAX * NWIN;                        // sorted entries
-constexpr uint32_t K1 = 16, KJ = 16;                                   // chunk lengths
-constexpr uint32_t T1_MAX = (uint32_t)((E_MAX + K1 - 1) / K1);
-constexpr uint32_t M2_MAX = 2 * T1_MAX;                                // level-1 partials
-constexpr uint32_t M3_MAX = 2 * ((M2_MAX + KJ - 1) / KJ);              // level-2 partials
+constexpr uint32_t FOLD_J = 4, FOLD_K = FOLD_QUADS * FOLD_J;           // leaves per quad and block
+constexpr uint32_t M2_MAX = 2 * (uint32_t)((E_MAX + FOLD_K - 1) / FOLD_K);  // level-1 partials
+constexpr uint32_t M3_MAX = 2 * ((M2_MAX + FOLD_K - 1) / FOLD_K);      // level-2 partials
 constexpr uint32_t RED_L = 8, RED_LOG2L = 3;
 constexpr uint32_t RED_NODES0 = NWIN * (BPW / RED_L);                  // 832
 constexpr int RED_LEVELS = 3;                                          // 512 -> 64 -> 8 -> 1
-constexpr int MAX_ACC_LEVELS = 16;
 constexpr size_t XS = sizeof(Xyzz<P>);
 
 constexpr size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -67,8 +65,7 @@ constexpr size_t OFF_COUNTS = 0;
 constexpr size_t OFF_CURSOR = align256(OFF_COUNTS + (NB + 1) * 4);
 constexpr size_t OFF_ENTS = align256(OFF_CURSOR + (NB + 1) * 4);
 constexpr size_t OFF_BUCKETS = align256(OFF_ENTS + E_MAX * 8);
-constexpr size_t OFF_CNT = align256(OFF_BUCKETS + NB * XS);
-constexpr size_t OFF_TILES = align256(OFF_CNT + T1_MAX * 4);
+constexpr size_t OFF_TILES = align256(OFF_BUCKETS + NB * XS);
 constexpr size_t OFF_TOTALS = align256(OFF_TILES + 4096);
 constexpr size_t OFF_PK0 = align256(OFF_TOTALS + 64 * 4);
 constexpr size_t OFF_PV0 = align256(OFF_PK0 + M2_MAX * 4);
@@ -83,7 +80,7 @@ constexpr size_t OFF_DESC = align256(OFF_PHI + (size_t)N_MAX * 2 * P::N * 4);
 constexpr size_t OFF_TASKS = align256(OFF_DESC + sizeof(MsmDesc));
 constexpr size_t SCRATCH_BYTES = align256(OFF_TASKS + RED_LEVELS * NWIN * sizeof(RedTask));
 static_assert(SCRATCH_BYTES < (16u << 20), "scratch must stay modest");
-static_assert((T1_MAX + 2047) / 2048 * 4 <= 4096, "scan tile sums fit their slot");
+static_assert((NB + 2047) / 2048 * 4 <= 4096, "scan tile sums fit their slot");
 
 static __device__ __align__(256) unsigned char g_scratch[SCRATCH_BYTES];
 
@@ -192,20 +189,6 @@ extern "C" ZkMetalStatus zkmsm_bn254_msm_noalloc(const void* d_points, const voi
         base = g_addr[dev];
     }
     const uint32_t n = n_points;
-    uint32_t accK[MAX_ACC_LEVELS], accT[MAX_ACC_LEVELS];
-    int nacc = 0;
-    uint64_t M = 2ull * n * NWIN;
-    uint32_t K = K1;
-    while (nacc < MAX_ACC_LEVELS) {
-        uint64_t T = (M + K - 1) / K;
-        if (T == 0) T = 1;
-        accK[nacc] = K;
-        accT[nacc] = (uint32_t)T;
-        nacc++;
-        if (T <= 1) break;
-        M = 2 * T;
-        K = KJ;
-    }
     k_noalloc_tables<<<1, 32, 0, s>>>(reinterpret_cast<MsmDesc*>(base + OFF_DESC),
                                       reinterpret_cast<RedTask*>(base + OFF_TASKS), n, (uint32_t)fmt);
     cudaError_t me = cudaMemsetAsync(base + OFF_COUNTS, 0, (NB + 1) * 4, s);
@@ -222,7 +205,6 @@ extern "C" ZkMetalStatus zkmsm_bn254_msm_noalloc(const void* d_points, const voi
     uint32_t* counts = reinterpret_cast<uint32_t*>(base + OFF_COUNTS);
     uint32_t* cursor = reinterpret_cast<uint32_t*>(base + OFF_CURSOR);
     uint2* ents = reinterpret_cast<uint2*>(base + OFF_ENTS);
-    uint32_t* cnt = reinterpret_cast<uint32_t*>(base + OFF_CNT);
     uint32_t* tot = reinterpret_cast<uint32_t*>(base + OFF_TOTALS);
     Xyzz<P>* buckets = reinterpret_cast<Xyzz<P>*>(base + OFF_BUCKETS);
     uint32_t* pk[2] = {reinterpret_cast<uint32_t*>(base + OFF_PK0), reinterpret_cast<uint32_t*>(base + OFF_PK1)};
@@ -236,22 +218,17 @@ extern "C" ZkMetalStatus zkmsm_bn254_msm_noalloc(const void* d_points, const voi
     k_digit_hist<C><<<(n + 255) / 256, 256, 0, s>>>(sc, dd, 1, n, counts);
     scan(base, counts, NB, tot + 0, cursor, s);
     k_digit_scatter<C><<<(n + 255) / 256, 256, 0, s>>>(sc, dd, 1, n, cursor, ents);
-    const uint32_t* lk = reinterpret_cast<const uint32_t*>(ents);
-    uint32_t ks = 2;
-    int cur = 0;
-    for (int l = 0; l < nacc; l++) {
-        uint32_t Kl = accK[l], Tl = accT[l];
-        k_chunk_count<<<(Tl + 255) / 256, 256, 0, s>>>(lk, ks, tot + l, Kl, Tl, cnt);
-        scan(base, cnt, Tl, tot + l + 1, nullptr, s);
+    uint64_t M = 2ull * n * NWIN;
+    for (int l = 0;; l++) {
+        const uint32_t T = (uint32_t)((M + FOLD_K - 1) / FOLD_K), c = l & 1;
         if (l == 0)
-            k_acc_l1<C><<<(Tl + AccLaunch<C>::THREADS - 1) / AccLaunch<C>::THREADS, AccLaunch<C>::THREADS, 0, s>>>(ents, tot + l, Kl, pts, phi, cnt, buckets, pk[cur],
-                                                          pv[cur]);
+            k_acc_fold<C, true><<<T, FOLD_THREADS, 0, s>>>(ents, pts, phi, nullptr, nullptr, tot, FOLD_J, T == 1,
+                                                           tot + 1, buckets, pk[c], pv[c]);
         else
-            k_acc_lj<C, false><<<(Tl + 255) / 256, 256, 0, s>>>(lk, pv[cur ^ 1], tot + l, Kl, cnt, buckets, pk[cur],
-                                                               pv[cur]);
-        lk = pk[cur];
-        ks = 1;
-        cur ^= 1;
+            k_acc_fold<C, false><<<T, FOLD_THREADS, 0, s>>>(nullptr, nullptr, nullptr, pk[c ^ 1], pv[c ^ 1], tot + l,
+                                                            FOLD_J, T == 1, tot + l + 1, buckets, pk[c], pv[c]);
+        if (T == 1) break;
+        M = 2ull * T;
     }
     const Xyzz<P>* inS = buckets;
     const Xyzz<P>* inW = nullptr;

@@ -234,8 +234,8 @@ struct Server {
                     double oldest = 0;
                     for (auto& r : batch)
                         oldest = std::max(oldest, std::chrono::duration<double, std::milli>(t_b0 - r->t_submit).count());
-                    const DevBuf* ws[] = {&eng->w_counts, &eng->w_cursor, &eng->w_ents, &eng->w_ents2,
-                                          &eng->w_thist, &eng->w_buckets, &eng->w_cnt, &eng->w_pkeys[0],
+                    const DevBuf* ws[] = {&eng->w_ents, &eng->w_ents2,
+                                          &eng->w_thist, &eng->w_buckets, &eng->w_pkeys[0],
                                           &eng->w_pkeys[1], &eng->w_pvals[0], &eng->w_pvals[1], &eng->w_redS[0],
                                           &eng->w_redS[1], &eng->w_redW[0], &eng->w_redW[1], &eng->w_tiles};
                     uint64_t wsb = d_cap;

@@ -88,6 +88,13 @@ constexpr uint32_t MSD_CHUNK_TILES = 8;
 constexpr uint32_t PROFILE_BINS = 320;
 constexpr uint32_t PROFILE_SAMPLES = 4096;
 
+// Segmented sums of the sorted entries (k_acc_fold): leaves per block are
+// FOLD_QUADS * J, J leaves per quad; entry sets up to ACC_FOLD_MAX_ENTRIES
+// skip the one-thread-per-chunk first level.
+constexpr uint32_t FOLD_THREADS = 256;
+constexpr uint32_t FOLD_QUADS = FOLD_THREADS / 4;
+constexpr uint64_t ACC_FOLD_MAX_ENTRIES = 1ull << 18;
+
 // Bucket-reduction levels with at most this many output nodes run the
 // inline-product kernel (few threads: latency-bound).
 constexpr uint32_t RED_INLINE_MAX_NODES = 32768;
