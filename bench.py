@@ -115,12 +115,15 @@ def plan_of(n, window=0, curve=0):
 
 
 def reduction_products(plan, curve="bn254"):
-    """Word products k_reduce_level executes over the plan's reduction tree: a
-    node of cnt children does 2(cnt - 1) + 1 XYZZ additions, cnt more above
-    level 0 (the weighted sums), and level * log2(L) doublings."""
+    """Word products of the bucket reduction's additions: in the levels of the
+    plan's tree that k_reduce_level runs, a node of cnt children does
+    2(cnt - 1) + 1 XYZZ additions, cnt more above level 0 (the weighted sums),
+    and level * log2(L) doublings; below them the quads' bit sums take two
+    additions per node."""
     L, lg = plan["red_L"], plan["red_log2L"]
-    adds = dbls = 0
-    for lvl, tasks in enumerate(plan["red"]):
+    quad = plan["quad"]
+    adds, dbls = 2 * sum(t[1] for t in quad["tasks"]), 0
+    for lvl, tasks in enumerate(plan["red"][:quad["levels"]]):
         for (_, n_in, _, _) in tasks:
             for cnt, k in ((L, n_in // L), (n_in % L, 1 if n_in % L else 0)):
                 adds += (2 * (cnt - 1) + 1 + (cnt if lvl else 0)) * k

@@ -350,7 +350,9 @@ ZkMetalStatus zkmsm_engine_phase_times(ZkMetalMSMEngine engine, double* ms5, uin
 
 /* The execution plan (window widths, bucket layout, chunking of the segmented
  * sums, reduction tree) the engine would use for a batch, as JSON text in
- * buf.  Pure host computation: no device is touched. */
+ * buf.  "red" is the whole reduction tree; its first "quad".levels levels run
+ * as such, and the windows' remaining nodes are "quad".tasks.  Pure host
+ * computation: no device is touched. */
 ZkMetalStatus zkmsm_plan_describe(int curve, const uint32_t* counts, uint32_t n_msms, int scalar_fmt,
                                   int window_bits, int chunk, int glv, int scalar_bits, char* buf, uint64_t buflen);
 /* The same for MSMs over prefixes of a table of table_points points with
@@ -400,7 +402,7 @@ ZkMetalStatus zkmsm_field_op(int curve, int op, const void* d_a, const void* d_b
  * n_points affine points (64 B), n_points scalars (32 B, scalar_fmt), result
  * 3 x 32 B (Jacobian, Z = 1 or the identity).  n_points <= 8192; larger ->
  * ZKMETAL_ERR_INVALID_INPUT.  Scratch is one static device array of about
- * 7.6 MB that every GPU loading the library holds until exit and that all
+ * 3.5 MB that every GPU loading the library holds until exit and that all
  * calls share: calls whose GPU work overlaps race, so serialise them (calls
  * queued one after another on one stream are already ordered).  The first
  * call on a device looks the array's address up and caches it (make that

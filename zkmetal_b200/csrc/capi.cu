@@ -1044,7 +1044,16 @@ static ZkMetalStatus plan_json(int curve, const uint32_t* counts, uint32_t n_msm
             }
             s += "]";
         }
-        s += "]}";
+        s += "],\"quad\":{\"levels\":" + std::to_string(pl.red_levels) + ",\"log2J\":" +
+             std::to_string(pl.quad_log2J) + ",\"log2E\":" + std::to_string(pl.quad_log2E) + ",\"blocks\":" +
+             std::to_string(pl.quad_blocks) + ",\"windows\":" + std::to_string(pl.quad_windows ? 1 : 0) +
+             ",\"tasks\":[";
+        for (size_t k = 0; k < pl.quad_tasks.size(); k++) {
+            auto& tk = pl.quad_tasks[k];
+            s += (k ? "," : "") + std::string("[") + std::to_string(tk.in_off) + "," + std::to_string(tk.n_in) + "," +
+                 std::to_string(tk.out_off) + "," + std::to_string(tk.n_out) + "]";
+        }
+        s += "]}}";
         if (s.size() + 1 > buflen) return ZKMETAL_ERR_INVALID_INPUT;
         memcpy(buf, s.c_str(), s.size() + 1);
         return ZKMETAL_SUCCESS;

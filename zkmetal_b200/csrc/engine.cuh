@@ -266,7 +266,14 @@ struct Plan {
     bool acc_fold = false;
     std::vector<uint32_t> acc_K, acc_T;
     std::vector<uint64_t> acc_Mbound;
-    // bucket-reduction levels
+    // bucket-reduction tree (levels of arity red_L to one node per window); the
+    // first red_levels of them run as kernels, and k_reduce_quads (quad_J =
+    // 2^quad_log2J nodes per quad, quad_tasks: one per window) and, when a
+    // window has several blocks, k_reduce_windows (2^quad_log2E blocks per
+    // quad) do the work of the rest
+    uint32_t red_levels = 0, quad_log2J = 0, quad_blocks = 0, quad_log2E = 0;
+    bool quad_windows = false;
+    std::vector<RedTask> quad_tasks;
     uint32_t red_L = 8, red_log2L = 3;
     // threads per block of the level-1 accumulation (0: the curve's default)
     uint32_t acc_threads = 0;
@@ -285,6 +292,9 @@ struct Plan {
         sort_maxd = sort_spb = sort_passes = sort_bits = sort_tiles = 0;
         msd_passes = msd_bits1 = msd_bits2 = msd_tiles1 = msd_tiles2 = 0;
         msd_groups1 = msd_chunks2 = 0;
+        red_levels = quad_log2J = quad_blocks = quad_log2E = 0;
+        quad_windows = false;
+        quad_tasks.clear();
         red_L = 8;
         red_log2L = 3;
         acc_threads = 0;
@@ -590,7 +600,7 @@ class Engine {
     DevBuf w_points, w_phi, w_scalars, w_ents, w_buckets;
     DevBuf w_ents2, w_thist, w_stripe_buckets, w_seg;
     DevBuf w_tiles, w_totals, w_pkeys[2], w_pvals[2], w_redS[2], w_redW[2];
-    DevBuf w_results, w_comb, w_profile;
+    DevBuf w_quad1, w_quad2, w_results, w_comb, w_profile;
     uint32_t* h_profile = nullptr;  // pinned, PROFILE_BINS words
     bool comb_ready[NCURVES] = {};
     uint32_t* h_results = nullptr;  // pinned
@@ -603,7 +613,7 @@ class Engine {
         DevBuf* bufs[] = {&w_points, &w_phi, &w_scalars, &w_ents, &w_buckets,
                           &w_ents2, &w_thist, &w_stripe_buckets, &w_seg, &w_tiles, &w_totals,
                           &w_pkeys[0], &w_pkeys[1], &w_pvals[0], &w_pvals[1], &w_redS[0], &w_redS[1],
-                          &w_redW[0], &w_redW[1], &w_results, &w_comb, &w_profile, &transient.d_descs,
+                          &w_redW[0], &w_redW[1], &w_quad1, &w_quad2, &w_results, &w_comb, &w_profile, &transient.d_descs,
                           &transient.d_tasks};
         for (DevBuf* b : bufs) b->sp = &stream;
         cudaMemPool_t pool;
@@ -908,6 +918,37 @@ class Engine {
             pl.red_tasks.push_back(nx);
             pl.red_nout.push_back(o);
         }
+        // the levels that run one thread per node, then the quads' blocks
+        std::vector<RedTask> wins;  // n_in nodes of each window from in_off
+        for (uint32_t lvl = 0;; lvl++) {
+            wins = pl.red_tasks[0];
+            uint64_t total = 0;
+            uint32_t most = 0;
+            for (size_t k = 0; k < wins.size(); k++) {
+                if (lvl) {
+                    wins[k].in_off = pl.red_tasks[lvl - 1][k].out_off;
+                    wins[k].n_in = pl.red_tasks[lvl - 1][k].n_out;
+                }
+                total += wins[k].n_in;
+                most = std::max(most, wins[k].n_in);
+            }
+            pl.red_levels = lvl;
+            if ((total <= RED_QUAD_MAX_NODES && most <= RED_QUAD_MAX_WINDOW) || lvl == pl.red_tasks.size()) {
+                pl.quad_log2J = most <= 8 * RED_QUADS ? 0 : 2;
+                break;
+            }
+        }
+        const uint32_t per = RED_QUADS << pl.quad_log2J;
+        uint32_t most_blocks = 1;
+        for (auto& t : wins) {
+            t.out_off = pl.quad_blocks;
+            t.n_out = (t.n_in + per - 1) / per;
+            pl.quad_blocks += t.n_out;
+            most_blocks = std::max(most_blocks, t.n_out);
+        }
+        pl.quad_windows = most_blocks > 1;
+        while ((8u << pl.quad_log2E) < most_blocks) pl.quad_log2E++;
+        pl.quad_tasks = std::move(wins);
     }
 
     // Plans are cached by shape, with their tables uploaded once, so that
@@ -955,6 +996,8 @@ class Engine {
             pl.task_level_off.push_back(blob.size());
             blob.insert(blob.end(), v.begin(), v.end());
         }
+        pl.task_level_off.push_back(blob.size());  // the quads' tasks last
+        blob.insert(blob.end(), pl.quad_tasks.begin(), pl.quad_tasks.end());
         pl.d_tasks.ensure((blob.size() + 1) * sizeof(RedTask));
         pl.d_descs.ensure((pl.descs.size() + 1) * sizeof(MsmDesc));
         if (async) {
@@ -1009,7 +1052,9 @@ class Engine {
             grew = true;
             ZK_CUDA(cudaMemsetAsync(w_totals.p, 0, 64 * 4, stream));
         }
-        size_t r0 = pl.red_nout.empty() ? 1 : pl.red_nout[0];
+        size_t r0 = pl.red_nout.empty() || !pl.red_levels ? 1 : pl.red_nout[0];
+        grew |= w_quad1.ensure((size_t)pl.quad_blocks * RED_SLOTS1 * xs + xs);
+        grew |= w_quad2.ensure((size_t)pl.nwin_total * RED_SLOTS2 * xs + xs);
         for (int i = 0; i < 2; i++) {
             grew |= w_redS[i].ensure(r0 * xs + xs);
             grew |= w_redW[i].ensure(r0 * xs + xs);

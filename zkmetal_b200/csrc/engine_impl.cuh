@@ -203,8 +203,8 @@ void Engine::enqueue(const Plan& pl, const uint32_t* d_bases, const uint32_t* d_
     prof_end(ev);
 }
 
-// Window sums from the buckets by a tree of running sums, then Horner over
-// the windows and affine normalisation into d_results.
+// Window sums from the buckets (running sums, then bit sums by quads), then
+// the windows' shifted sum and affine normalisation into d_results.
 template <class C>
 void Engine::enqueue_reduce(const Plan& pl, const void* bucket_base, uint32_t* d_results,
                             std::vector<cudaEvent_t>* ev) {
@@ -214,28 +214,42 @@ void Engine::enqueue_reduce(const Plan& pl, const void* bucket_base, uint32_t* d
     const Xyzz<P>* inS = static_cast<const Xyzz<P>*>(bucket_base);
     const Xyzz<P>* inW = nullptr;
     int rc = 0;
-    for (size_t l = 0; l < pl.red_tasks.size(); l++) {
+    for (size_t l = 0; l < pl.red_levels; l++) {
         uint32_t nout = pl.red_nout[l];
         const RedTask* tk = pl.d_tasks.as<RedTask>() + pl.task_level_off[l];
         Xyzz<P>* oS = w_redS[rc].as<Xyzz<P>>();
         Xyzz<P>* oW = w_redW[rc].as<Xyzz<P>>();
-        if (nout <= RED_INLINE_MAX_NODES)
-            k_reduce_level<C, true><<<(nout + 127) / 128, 128, 0, stream>>>(inS, inW, tk, (int)pl.red_tasks[l].size(),
-                                                                           nout, pl.red_L,
-                                                                           (uint32_t)l * pl.red_log2L, oS, oW);
-        else
-            k_reduce_level<C, false><<<(nout + 127) / 128, 128, 0, stream>>>(
-                    inS, inW, tk, (int)pl.red_tasks[l].size(), nout, pl.red_L, (uint32_t)l * pl.red_log2L, oS, oW);
+        k_reduce_level<C><<<(nout + 127) / 128, 128, 0, stream>>>(inS, inW, tk, (int)pl.red_tasks[l].size(), nout,
+                                                                 pl.red_L, (uint32_t)l * pl.red_log2L, oS, oW);
         launches++;
         ZK_CUDA(cudaGetLastError());
         inS = oS;
         inW = oW;
         rc ^= 1;
     }
+    const RedTask* qt = pl.d_tasks.as<RedTask>() + pl.task_level_off.back();
+    const uint32_t nw = (uint32_t)pl.quad_tasks.size(), span = pl.red_levels * pl.red_log2L;
+    CombineTerms ct{RED_SLOTS1, span + pl.quad_log2J, 0, 0};
+    Xyzz<P>* terms = w_quad1.as<Xyzz<P>>();
+    if (pl.quad_blocks) {
+        k_reduce_quads<C><<<pl.quad_blocks, 4 * RED_QUADS, 0, stream>>>(inS, inW, qt, (int)nw, 1u << pl.quad_log2J, span,
+                                                                       terms);
+        launches++;
+        ZK_CUDA(cudaGetLastError());
+    }
+    if (pl.quad_windows) {
+        k_reduce_windows<C><<<nw, 32 * RED_SLOTS1, 0, stream>>>(terms, qt, 1u << pl.quad_log2E, w_quad2.as<Xyzz<P>>());
+        launches++;
+        ZK_CUDA(cudaGetLastError());
+        terms = w_quad2.as<Xyzz<P>>();
+        ct.slots = RED_SLOTS2;
+        ct.bit_x = ct.bit_t + 6;  // log2(RED_QUADS) bits of T
+        ct.bit_t2 = ct.bit_x + pl.quad_log2E;
+    }
     if (ev) prof_mark(*ev, 4);
     uint32_t most = 1;
     for (const auto& d : pl.descs) most = std::max(most, d.nred);
-    k_combine<C><<<nd, combine_threads(most), 0, stream>>>(inS, inW, dd, nd, d_results);
+    k_combine<C><<<nd, combine_threads(most), 0, stream>>>(terms, ct, dd, nd, d_results);
     launches++;
     ZK_CUDA(cudaGetLastError());
     if (ev) prof_mark(*ev, 5);

@@ -25,10 +25,12 @@
 //                     tree per block, repeated until one block is left
 //                     (handles any skew, e.g. 20% of all points in one bucket
 //                     for witness scalars).
-//  6. k_reduce_level  per window sum_b b*B_b by a tree of running sums.
+//  6. k_reduce_level, k_reduce_quads, k_reduce_windows
+//                     per window sum_b b*B_b: running sums while there are
+//                     many nodes, then bit sums by quads of lanes.
 //                     [msm_kernels.metal:152-248]
-//  7. k_combine       sum of the windows shifted to their bit offsets (a
-//                     quad of lanes per window), normalise to affine.
+//  7. k_combine       the windows' bit sums shifted into place (quads of
+//                     lanes), normalise to affine.
 //                     [MSMEngine.swift:899-904, msm_kernels.metal:251-275]
 #pragma once
 #include "quad.cuh"
@@ -1143,10 +1145,18 @@ __global__ void __launch_bounds__(FOLD_THREADS) k_acc_fold(const uint2* __restri
 // ------------------------------------------------------------ bucket reduction
 //
 // A window's sum is sum_{b=1..B} b*B_b = sum_i (i+1) A_i with A_i = B_{i+1}.
-// Each tree node over a bucket range keeps S = sum A_i and W = sum (i - lo) A_i.
+// A node over a bucket range keeps S = sum A_i and W = sum (i - lo) A_i.
 // Merging L children of span `span`: S' = sum S_s and
 // W' = sum W_s + span * sum_s s*S_s, the last sum by a running sum.
-// At the root: window sum = W + S.
+// k_reduce_level does that with one thread per node while the nodes fill the
+// multiply pipe.  With fewer nodes a chain of 2L additions in one thread
+// costs 8.7 us an addition (BN254), 180-200 us a level whatever its size (BN254
+// 2^20: 907 us for five levels; now 146 us for the first, 69 + 23 us for the
+// quads; 2^16: 365 us for three, now 27 + 16), so the rest of the tree goes to quads of lanes and to plain sums instead:
+// sum_i i*S_i = sum_j 2^j T_j, T_j the sum of the S_i whose index has bit j
+// set, all of them by-products of one tree of depth log2(nodes)
+// (k_reduce_quads, k_reduce_windows), and k_combine shifts the T_j into place
+// on its chain of doublings, which passes those bits anyway.
 
 ZK_DEV int find_task(const RedTask* __restrict__ t, int nt, uint32_t g) {
     int lo = 0, hi = nt - 1;
@@ -1158,9 +1168,7 @@ ZK_DEV int find_task(const RedTask* __restrict__ t, int nt, uint32_t g) {
     return lo;
 }
 
-// INL: inline products, for the top levels, whose few threads are
-// latency-bound (a lone thread's out-of-line products cannot overlap).
-template <class C, bool INL>
+template <class C>
 __global__ void __launch_bounds__(128) k_reduce_level(const Xyzz<typename C::Fp>* __restrict__ inS,
                                                       const Xyzz<typename C::Fp>* __restrict__ inW,
                                                       const RedTask* __restrict__ tasks, int ntasks,
@@ -1180,52 +1188,212 @@ __global__ void __launch_bounds__(128) k_reduce_level(const Xyzz<typename C::Fp>
 #pragma unroll 1
     for (int s = (int)cnt - 1; s >= 1; s--) {
         load_xyzz(q, inS + c0 + s);
-        xyzz_add<P, INL>(run, q);
-        xyzz_add<P, INL>(x, run);
+        xyzz_add(run, q);
+        xyzz_add(x, run);
     }
     load_xyzz(q, inS + c0);
-    xyzz_add<P, INL>(run, q);
+    xyzz_add(run, q);
     store_xyzz(outS + g, run);
 #pragma unroll 1
-    for (uint32_t d = 0; d < log2span; d++) xyzz_dbl<P, INL>(x, x);
+    for (uint32_t d = 0; d < log2span; d++) xyzz_dbl(x, x);
     if (inW != nullptr) {
 #pragma unroll 1
         for (uint32_t s = 0; s < cnt; s++) {
             load_xyzz(q, inW + c0 + s);
-            xyzz_add<P, INL>(x, q);
+            xyzz_add(x, q);
         }
     }
     store_xyzz(outW + g, x);
 }
 
-// Window combine, one block per MSM: R = sum_w 2^bit(w) * (S_w + W_w).  Quad
-// w owns window w: it forms T_w = S_w + W_w, doubles it bit(w) times, and a
-// tree through shared memory adds the quads' points; quad 0 normalises to
-// affine and writes the reference-layout Jacobian (X, Y, Z) Montgomery with
-// Z = 1 (or the identity (1, 1, 0)).
-//
-// Latency-bound: one chain of as many doublings as the top window's bit
-// offset (BN254: up to 124), log2(windows) additions and one inversion,
-// whatever n is.  A quad (quad.cuh) runs a doubling in two product layers, so
-// the chain is about 250 product times; the top windows' warps run alone on
-// their schedulers up to 32 windows (four warps).  At 2^8 points (BN254, 32
-// windows) 234 us, 2^17 BLS12-377 419 us, 2^16 BN254 G2 723 us, against 378,
-// 885 and 1034 us when four warps shared the three layers of XYZZ doublings
-// through shared memory and a binary Euclid inverted.
-// Up to 64 windows; a shift-table MSM has one window sum and no doublings.
+// One step of the tree over the quads of a warp (st < 8) or a block: quad i
+// holds S of the nodes it stands for, and w, a plain sum.  Quad i with bit st
+// clear and at most one lower bit set adds the S of quad i + st: no lower bit
+// set continues the sum of all S, bit j alone continues T_j (whose terms are
+// the S that quads with bit j set held at step j).  The w's travel to the
+// quad whose lower bits are all set: quad i with bit st set and all lower
+// bits set adds quad i - st's w.  So a quad does one addition at most.
+template <class P>
+ZK_DEV void reduce_step(Fe<P>& S, Fe<P>& w, uint32_t i, uint32_t st, uint32_t q, const Fe<P>& got) {
+    const uint32_t low = i & (st - 1);
+    const bool up = i & st;
+    const bool on = up ? low == st - 1 : (low & (low - 1)) == 0;
+    Fe<P> a, b;
+    fe_select(a, up, w, S);
+    fe_set_zero(b);
+    fe_select(b, on, got, b);
+    quad_add(a, b, q);
+    fe_select(w, up, a, w);
+    fe_select(S, up, S, a);
+}
 
-// threads of k_combine for MSMs of at most `windows` window sums
-inline uint32_t combine_threads(uint32_t windows) { return windows < 8 ? 32u : (4 * windows + 31) / 32 * 32; }
+// What the partner of quad i at this step needs: its S from above, w from below.
+template <class P>
+ZK_DEV void reduce_swap(Fe<P>& got, const Fe<P>& S, const Fe<P>& w, uint32_t i, uint32_t st) {
+    Fe<P> send;
+    fe_select(send, (i & st) != 0, S, w);
+#pragma unroll
+    for (int l = 0; l < P::N; l++) got.v[l] = __shfl_xor_sync(0xffffffffu, send.v[l], 4 * st);
+}
+
+// The nodes of every window (tasks: one per window, n_out blocks each from
+// block out_off) in blocks of RED_QUADS * J; quad i sums nodes [i*J, (i+1)*J)
+// by a running sum, x = sum s*S_s shifted by the nodes' span (2^log2span) and
+// added to the nodes' W, then log2(quads) tree steps.  Block b writes
+// RED_SLOTS1 points: S | T_0 .. T_5 | W, with the window's sum =
+// S + W + sum_j 2^(log2span + log2J + j) T_j when it is one block.
+template <class C>
+__global__ void __launch_bounds__(4 * RED_QUADS) k_reduce_quads(const Xyzz<typename C::Fp>* __restrict__ inS,
+                                                                const Xyzz<typename C::Fp>* __restrict__ inW,
+                                                                const RedTask* __restrict__ tasks, int ntasks,
+                                                                uint32_t J, uint32_t log2span,
+                                                                Xyzz<typename C::Fp>* __restrict__ out) {
+    using P = typename C::Fp;
+    __shared__ uint4 sh_raw[RED_QUADS * sizeof(Xyzz<P>) / sizeof(uint4)];
+    Xyzz<P>* sh = reinterpret_cast<Xyzz<P>*>(sh_raw);
+    const uint32_t i = threadIdx.x >> 2, q = threadIdx.x & 3;
+    const RedTask tk = tasks[find_task(tasks, ntasks, blockIdx.x)];
+    const uint32_t n0 = (blockIdx.x - tk.out_off) * RED_QUADS * J;
+    const uint32_t cnt = min(RED_QUADS * J, tk.n_in - n0);  // nodes of this block
+    const uint32_t base = tk.in_off + n0 + i * J, mine = cnt > i * J ? min(J, cnt - i * J) : 0u;
+    Fe<P> run, x, v;
+    fe_set_zero(run);
+    fe_set_zero(x);
+#pragma unroll 1
+    for (uint32_t s = J; s-- > 0;) {
+        fe_set_zero(v);
+        if (s < mine) quad_load(v, inS + base + s, q);
+        quad_add(run, v, q);
+        if (s) quad_add(x, run, q);
+    }
+    if (inW != nullptr) {
+        if (J > 1)
+#pragma unroll 1
+            for (uint32_t d = 0; d < log2span; d++) quad_dbl(x, q);
+#pragma unroll 1
+        for (uint32_t s = 0; s < J; s++) {
+            fe_set_zero(v);
+            if (s < mine) quad_load(v, inW + base + s, q);
+            quad_add(x, v, q);
+        }
+    }
+    const uint32_t used = (cnt + J - 1) / J;  // quads with nodes
+    uint32_t st = 1;
+#pragma unroll 1
+    for (; st < used; st <<= 1) {
+        if (st < 8) {
+            reduce_swap(v, run, x, i, st);
+        } else {
+            fe_select(v, (i & st) != 0, run, x);
+            quad_store(sh + i, v, q);
+            __syncthreads();
+            quad_load(v, sh + (i ^ st), q);
+            __syncthreads();
+        }
+        reduce_step(run, x, i, st, q, v);
+    }
+    // S in quad 0, T_j in quad 2^j below st (none above), W in quad st - 1
+    Xyzz<P>* o = out + (size_t)blockIdx.x * RED_SLOTS1;
+    if (i == 0) quad_store(o, run, q);
+    if (i && !(i & (i - 1))) {
+        if (i >= st) fe_set_zero(run);
+        quad_store(o + __ffs(i), run, q);
+    }
+    if (i == st - 1) quad_store(o + RED_SLOTS1 - 1, x, q);
+}
+
+// Windows of more than one block: one block per window, warp a sums slot a of
+// the window's blocks (quad i: blocks [i*E, (i+1)*E), then three tree steps);
+// the S of the blocks give three more bit sums and X = sum over quads of
+// their running sums.  Writes RED_SLOTS2 points: S | T_0 .. T_5 | W | X |
+// T'_0 .. T'_2, X and T'_j at bits log2block and log2block + log2E + j.
+template <class C>
+__global__ void __launch_bounds__(32 * RED_SLOTS1) k_reduce_windows(const Xyzz<typename C::Fp>* __restrict__ in,
+                                                                    const RedTask* __restrict__ tasks, uint32_t E,
+                                                                    Xyzz<typename C::Fp>* __restrict__ out) {
+    using P = typename C::Fp;
+    const uint32_t a = threadIdx.x >> 5, i = (threadIdx.x >> 2) & 7, q = threadIdx.x & 3;
+    const RedTask tk = tasks[blockIdx.x];
+    Fe<P> run, x, v;
+    fe_set_zero(run);
+    fe_set_zero(x);
+#pragma unroll 1
+    for (uint32_t s = E; s-- > 0;) {
+        const uint32_t b = i * E + s;
+        fe_set_zero(v);
+        if (b < tk.n_out) quad_load(v, in + (size_t)(tk.out_off + b) * RED_SLOTS1 + a, q);
+        if (a == 0) {  // warp-uniform
+            quad_add(run, v, q);
+            if (s) quad_add(x, run, q);
+        } else {
+            quad_add(x, v, q);
+        }
+    }
+#pragma unroll 1
+    for (uint32_t st = 1; st < 8; st <<= 1) {
+        reduce_swap(v, run, x, i, st);
+        reduce_step(run, x, i, st, q, v);
+    }
+    Xyzz<P>* o = out + (size_t)blockIdx.x * RED_SLOTS2;
+    if (a == 0) {
+        if (i == 0) quad_store(o, run, q);
+        if (i && !(i & (i - 1))) quad_store(o + RED_SLOTS1 + __ffs(i), run, q);
+        if (i == 7) quad_store(o + RED_SLOTS1, x, q);
+    } else if (i == 7) {
+        quad_store(o + a, x, q);
+    }
+}
+
+// Window combine, one block per MSM: R = sum over windows w and terms t of
+// 2^(bit(w) + bit(t)) * term, the terms being the points k_reduce_quads or
+// k_reduce_windows left per window, in order of their bits.  Each window's
+// terms go to COMBINE_SPLIT(windows) quads, neighbouring terms together; a
+// quad adds its terms up by Horner's rule and doubles the sum down to bit 0,
+// a tree through shared memory adds the quads' points, and quad 0 normalises
+// to affine and writes the reference-layout Jacobian (X, Y, Z) Montgomery
+// with Z = 1 (or the identity (1, 1, 0)).
+//
+// Latency-bound: one chain of as many doublings as the highest bit (BN254:
+// 127), a few additions and one inversion, whatever n is.  A quad (quad.cuh)
+// runs a doubling in two product layers, so the chain is about 250 product
+// times.  Four warps (32 quads) have a scheduler each; more would queue for
+// the multiply pipe, hence the split.  With the bit sums' Horner steps 266 us
+// at 2^8 points (BN254, 32 windows) and 262 us at 2^16 (11 windows), BLS12-377
+// 10^5 487 us, BN254 G2 2^16 844 us; four warps sharing the layers of XYZZ
+// doublings through shared memory, with a binary Euclid and without those
+// steps, took 378, 434, 885 and 1034 us.
+struct CombineTerms {
+    uint32_t slots;     // points per window: RED_SLOTS1 or RED_SLOTS2
+    uint32_t bit_t;     // bit of T_0
+    uint32_t bit_x;     // RED_SLOTS2: bit of X, and of T'_0
+    uint32_t bit_t2;
+};
+
+// quads per window
+__host__ __device__ inline uint32_t combine_split(uint32_t windows) {
+    return windows <= 8 ? 4 : windows <= 16 ? 2 : 1;
+}
+// threads of k_combine for MSMs of at most `windows` windows (the splits of
+// fewer windows need no more quads than 32 or `windows`)
+inline uint32_t combine_threads(uint32_t windows) {
+    const uint32_t quads = windows * combine_split(windows);
+    return windows > 1 && quads < 32 ? 128u : (4 * quads + 31) / 32 * 32;
+}
+
+// term at position k in order of bits: its slot and its bit in the window
+ZK_DEV uint32_t term_slot(uint32_t k) { return k == 0 ? 0 : k == 1 ? RED_SLOTS1 - 1 : k < RED_SLOTS1 ? k - 1 : k; }
+ZK_DEV uint32_t term_bit(uint32_t k, const CombineTerms& ct) {
+    return k < 2 ? 0 : k < RED_SLOTS1 ? ct.bit_t + k - 2 : k == RED_SLOTS1 ? ct.bit_x : ct.bit_t2 + k - RED_SLOTS1 - 1;
+}
 
 template <class C>
-__global__ void __launch_bounds__(4 * MAX_WINDOWS) k_combine(const Xyzz<typename C::Fp>* __restrict__ rootS,
-                                                             const Xyzz<typename C::Fp>* __restrict__ rootW,
-                                                             const MsmDesc* __restrict__ descs, int nd,
-                                                             uint32_t* __restrict__ out) {
+__global__ void __launch_bounds__(4 * MAX_WINDOWS) k_combine(const Xyzz<typename C::Fp>* __restrict__ terms,
+                                                             CombineTerms ct, const MsmDesc* __restrict__ descs,
+                                                             int nd, uint32_t* __restrict__ out) {
     using P = typename C::Fp;
     __shared__ uint4 sh_raw[MAX_WINDOWS * sizeof(Xyzz<P>) / sizeof(uint4)];
     Xyzz<P>* sh = reinterpret_cast<Xyzz<P>*>(sh_raw);
-    const uint32_t w = threadIdx.x >> 2, q = threadIdx.x & 3, warp = threadIdx.x >> 5;
+    const uint32_t u = threadIdx.x >> 2, q = threadIdx.x & 3, warp = threadIdx.x >> 5;
     const int m = (int)blockIdx.x;
     if (m >= nd) return;  // block-uniform
     const MsmDesc d = descs[m];
@@ -1237,35 +1405,50 @@ __global__ void __launch_bounds__(4 * MAX_WINDOWS) k_combine(const Xyzz<typename
             for (int l = 0; l < P::N; l++) { o[l] = one.v[l]; o[P::N + l] = one.v[l]; o[2 * P::N + l] = 0; }
         return;
     }
-    const uint32_t nw = d.nred;
+    const uint32_t split = combine_split(d.nred), nq = d.nred * split;  // quads in use
+    const uint32_t w = u / split, per = ct.slots / split;
+    const uint32_t lo = (u % split) * per;  // this quad's terms: positions [lo, lo + per)
+    const bool live = u < nq;
+    const Xyzz<P>* wt = terms + (size_t)(d.win_off + w) * ct.slots;
     Fe<P> a, b;
     fe_set_zero(a);
-    fe_set_zero(b);
-    if (w < nw) {
-        quad_load(a, rootS + d.win_off + w, q);
-        quad_load(b, rootW + d.win_off + w, q);
-    }
-    quad_add(a, b, q);
-    // bit(w) doublings; a warp runs to the most of its quads
-    const uint32_t cnt = w < nw ? win_bit(d, w) : 0u;
-    const uint32_t most = __reduce_max_sync(0xffffffffu, cnt);
-    if (most) {
-        QuadChain<C>::enter(a, q);
+    if (8 * warp < nq) {  // warp-uniform
+        if (live) quad_load(a, wt + term_slot(lo + per - 1), q);
 #pragma unroll 1
-        for (uint32_t i = 0; i < most; i++) {
-            b = a;
-            QuadChain<C>::dbl(b, q);
-            fe_select(a, i < cnt, b, a);
-        }
-        QuadChain<C>::leave(a, q);
-    }
-    for (uint32_t st = 1; st < nw; st <<= 1) {
-        // quads w with bits below st clear hold the sums of [w, w + st)
-        if (w & st && !(w & (st - 1))) quad_store(sh + w, a, q);
-        __syncthreads();
-        if (8 * warp < nw) {  // warp-uniform
+        for (uint32_t k = per - 1; k-- > 0;) {
+            const uint32_t cnt = live ? term_bit(lo + k + 1, ct) - term_bit(lo + k, ct) : 0u;
+            const uint32_t most = __reduce_max_sync(0xffffffffu, cnt);
+#pragma unroll 1
+            for (uint32_t i = 0; i < most; i++) {
+                b = a;
+                quad_dbl(b, q);
+                fe_select(a, i < cnt, b, a);
+            }
             fe_set_zero(b);
-            if (!(w & (2 * st - 1)) && w + st < nw) quad_load(b, sh + w + st, q);
+            if (live) quad_load(b, wt + term_slot(lo + k), q);
+            quad_add(a, b, q);
+        }
+        // down to bit 0; a warp runs to the most of its quads
+        const uint32_t cnt = live ? win_bit(d, w) + term_bit(lo, ct) : 0u;
+        const uint32_t most = __reduce_max_sync(0xffffffffu, cnt);
+        if (most) {
+            QuadChain<C>::enter(a, q);
+#pragma unroll 1
+            for (uint32_t i = 0; i < most; i++) {
+                b = a;
+                QuadChain<C>::dbl(b, q);
+                fe_select(a, i < cnt, b, a);
+            }
+            QuadChain<C>::leave(a, q);
+        }
+    }
+    for (uint32_t st = 1; st < nq; st <<= 1) {
+        // quads u with bits below st clear hold the sums of [u, u + st)
+        if (u & st && !(u & (st - 1))) quad_store(sh + u, a, q);
+        __syncthreads();
+        if (8 * warp < nq) {  // warp-uniform
+            fe_set_zero(b);
+            if (!(u & (2 * st - 1)) && u + st < nq) quad_load(b, sh + u + st, q);
             quad_add(a, b, q);
         }
         __syncthreads();

@@ -12,7 +12,7 @@
 // How: all scratch (bucket counts, sorted entries, buckets, partial sums,
 // reduction nodes, the endomorphism image of the bases, the launch tables)
 // lives in one file-scope __device__ array g_scratch of SCRATCH_BYTES
-// (7,572,224 bytes),
+// (3,486,976 bytes),
 // which every GPU that loads the library holds until the process exits.
 // Host code cannot use the array's name as a device address, so the first
 // call on each device (with that device current) looks its address up with
@@ -53,9 +53,8 @@ constexpr uint64_t E_MAX = 2ull * N_MAX * NWIN;                        // sorted
 constexpr uint32_t FOLD_J = 4, FOLD_K = FOLD_QUADS * FOLD_J;           // leaves per quad and block
 constexpr uint32_t M2_MAX = 2 * (uint32_t)((E_MAX + FOLD_K - 1) / FOLD_K);  // level-1 partials
 constexpr uint32_t M3_MAX = 2 * ((M2_MAX + FOLD_K - 1) / FOLD_K);      // level-2 partials
-constexpr uint32_t RED_L = 8, RED_LOG2L = 3;
-constexpr uint32_t RED_NODES0 = NWIN * (BPW / RED_L);                  // 832
-constexpr int RED_LEVELS = 3;                                          // 512 -> 64 -> 8 -> 1
+constexpr uint32_t RED_NB = BPW / RED_QUADS;                           // reduction blocks per window
+static_assert(RED_NB <= 8 && RED_NB * RED_QUADS == BPW, "a window's blocks fit one warp's quads");
 constexpr size_t XS = sizeof(Xyzz<P>);
 
 constexpr size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -71,14 +70,12 @@ constexpr size_t OFF_PK0 = align256(OFF_TOTALS + 64 * 4);
 constexpr size_t OFF_PV0 = align256(OFF_PK0 + M2_MAX * 4);
 constexpr size_t OFF_PK1 = align256(OFF_PV0 + M2_MAX * XS);
 constexpr size_t OFF_PV1 = align256(OFF_PK1 + M3_MAX * 4);
-constexpr size_t OFF_RS0 = align256(OFF_PV1 + M3_MAX * XS);
-constexpr size_t OFF_RW0 = align256(OFF_RS0 + RED_NODES0 * XS);
-constexpr size_t OFF_RS1 = align256(OFF_RW0 + RED_NODES0 * XS);
-constexpr size_t OFF_RW1 = align256(OFF_RS1 + RED_NODES0 * XS);
-constexpr size_t OFF_PHI = align256(OFF_RW1 + RED_NODES0 * XS);
+constexpr size_t OFF_Q1 = align256(OFF_PV1 + M3_MAX * XS);
+constexpr size_t OFF_Q2 = align256(OFF_Q1 + NWIN * RED_NB * RED_SLOTS1 * XS);
+constexpr size_t OFF_PHI = align256(OFF_Q2 + NWIN * RED_SLOTS2 * XS);
 constexpr size_t OFF_DESC = align256(OFF_PHI + (size_t)N_MAX * 2 * P::N * 4);
 constexpr size_t OFF_TASKS = align256(OFF_DESC + sizeof(MsmDesc));
-constexpr size_t SCRATCH_BYTES = align256(OFF_TASKS + RED_LEVELS * NWIN * sizeof(RedTask));
+constexpr size_t SCRATCH_BYTES = align256(OFF_TASKS + NWIN * sizeof(RedTask));
 static_assert(SCRATCH_BYTES < (16u << 20), "scratch must stay modest");
 static_assert((NB + 2047) / 2048 * 4 <= 4096, "scan tile sums fit their slot");
 
@@ -89,7 +86,7 @@ static unsigned char* g_addr[64];
 
 // The launch tables of one call, built on the device from by-value
 // arguments: the MSM descriptor (one MSM, window width CB, GLV) and the
-// reduction tasks (RED_LEVELS levels of NWIN windows, L = RED_L).
+// reduction tasks (one per window).
 static __global__ void k_noalloc_tables(MsmDesc* __restrict__ desc, RedTask* __restrict__ tasks, uint32_t n,
                                         uint32_t fmt) {
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
@@ -107,19 +104,7 @@ static __global__ void k_noalloc_tables(MsmDesc* __restrict__ desc, RedTask* __r
     d.nred = NWIN;
     d.nlo = NWIN;
     *desc = d;
-    uint32_t nin = BPW;
-    for (int l = 0; l < RED_LEVELS; l++) {
-        const uint32_t nout = (nin + RED_L - 1) / RED_L;
-        for (uint32_t w = 0; w < NWIN; w++) {
-            RedTask t;
-            t.in_off = l == 0 ? w * BPW : w * nin;
-            t.n_in = nin;
-            t.out_off = w * nout;
-            t.n_out = nout;
-            tasks[l * NWIN + w] = t;
-        }
-        nin = nout;
-    }
+    for (uint32_t w = 0; w < NWIN; w++) tasks[w] = RedTask{w * BPW, BPW, w * RED_NB, RED_NB};
 }
 
 static void scan(unsigned char* base, uint32_t* d, uint32_t n, uint32_t* d_total, uint32_t* copy, cudaStream_t s) {
@@ -209,8 +194,6 @@ extern "C" ZkMetalStatus zkmsm_bn254_msm_noalloc(const void* d_points, const voi
     Xyzz<P>* buckets = reinterpret_cast<Xyzz<P>*>(base + OFF_BUCKETS);
     uint32_t* pk[2] = {reinterpret_cast<uint32_t*>(base + OFF_PK0), reinterpret_cast<uint32_t*>(base + OFF_PK1)};
     Xyzz<P>* pv[2] = {reinterpret_cast<Xyzz<P>*>(base + OFF_PV0), reinterpret_cast<Xyzz<P>*>(base + OFF_PV1)};
-    Xyzz<P>* rS[2] = {reinterpret_cast<Xyzz<P>*>(base + OFF_RS0), reinterpret_cast<Xyzz<P>*>(base + OFF_RS1)};
-    Xyzz<P>* rW[2] = {reinterpret_cast<Xyzz<P>*>(base + OFF_RW0), reinterpret_cast<Xyzz<P>*>(base + OFF_RW1)};
     const MsmDesc* dd = reinterpret_cast<const MsmDesc*>(base + OFF_DESC);
     const RedTask* dt = reinterpret_cast<const RedTask*>(base + OFF_TASKS);
 
@@ -230,18 +213,13 @@ extern "C" ZkMetalStatus zkmsm_bn254_msm_noalloc(const void* d_points, const voi
         if (T == 1) break;
         M = 2ull * T;
     }
-    const Xyzz<P>* inS = buckets;
-    const Xyzz<P>* inW = nullptr;
-    uint32_t nodes = BPW;
-    for (int l = 0; l < RED_LEVELS; l++) {
-        nodes = (nodes + RED_L - 1) / RED_L;
-        uint32_t nout = nodes * NWIN;
-        k_reduce_level<C, false><<<(nout + 127) / 128, 128, 0, s>>>(inS, inW, dt + l * NWIN, NWIN, nout, RED_L,
-                                                             (uint32_t)l * RED_LOG2L, rS[l & 1], rW[l & 1]);
-        inS = rS[l & 1];
-        inW = rW[l & 1];
-    }
-    k_combine<C><<<1, combine_threads(NWIN), 0, s>>>(inS, inW, dd, 1, static_cast<uint32_t*>(d_result));
+    // 512 buckets per window: one node per quad, then the windows' blocks
+    Xyzz<P>* q1 = reinterpret_cast<Xyzz<P>*>(base + OFF_Q1);
+    Xyzz<P>* q2 = reinterpret_cast<Xyzz<P>*>(base + OFF_Q2);
+    k_reduce_quads<C><<<NWIN * RED_NB, 4 * RED_QUADS, 0, s>>>(buckets, nullptr, dt, NWIN, 1, 0, q1);
+    k_reduce_windows<C><<<NWIN, 32 * RED_SLOTS1, 0, s>>>(q1, dt, 1, q2);
+    k_combine<C><<<1, combine_threads(NWIN), 0, s>>>(q2, CombineTerms{RED_SLOTS2, 0, 6, 6}, dd, 1,
+                                                     static_cast<uint32_t*>(d_result));
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         set_error(std::string("zkmsm_bn254_msm_noalloc: launch failed: ") + cudaGetErrorString(e));

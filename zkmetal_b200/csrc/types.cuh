@@ -95,9 +95,14 @@ constexpr uint32_t FOLD_THREADS = 256;
 constexpr uint32_t FOLD_QUADS = FOLD_THREADS / 4;
 constexpr uint64_t ACC_FOLD_MAX_ENTRIES = 1ull << 18;
 
-// Bucket-reduction levels with at most this many output nodes run the
-// inline-product kernel (few threads: latency-bound).
-constexpr uint32_t RED_INLINE_MAX_NODES = 32768;
+// Bucket reduction: one-thread-per-node levels (k_reduce_level) run while
+// there are more than RED_QUAD_MAX_NODES nodes in all or RED_QUAD_MAX_WINDOW
+// in a window; k_reduce_quads takes the rest, one node per quad while the
+// windows fit eight such blocks, else four.
+constexpr uint32_t RED_QUAD_MAX_NODES = 65536;
+constexpr uint32_t RED_QUAD_MAX_WINDOW = 16384;
+constexpr uint32_t RED_QUADS = 64;                       // quads per block
+constexpr uint32_t RED_SLOTS1 = 8, RED_SLOTS2 = 12;      // points per block / per window
 
 struct RedTask {
     uint32_t in_off;   // first child node
