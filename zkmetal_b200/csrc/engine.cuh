@@ -332,18 +332,25 @@ inline int nearest_log2(uint64_t n) {
 // Signed windows a half-scalar of `bits` bits needs at width c.
 inline uint32_t windows_for(uint32_t bits, uint32_t c) { return (bits + 1 + c - 1) / c; }
 
-// Relative cost of window width c for `entries_per_window` entries: mixed
-// additions (one per nonzero digit) plus ~3 XYZZ additions per bucket in the
-// reduction, plus a latency term for the reduction depth and Horner chain.
+// Window width for `entries_per_window` entries per window, by a cost in
+// units of one mixed addition of a busy device (0.16 ns, BN254): an entry each
+// -- up to two while there are few, whose sums are chains of additions rather
+// than throughput -- about four per bucket, a one-thread-per-node reduction
+// level (some 150 us) when the buckets are too many for the quads alone, and
+// 8 us per bit of width for the reduction's and the combine's additions.  The
+// number of doublings does not depend on the width.  Measured best widths
+// (BN254): 2^8 points 4 (402 us; 5: 425), 2^10 4-8 (445-457), 2^12 7-10
+// (500-514; 5: 514), 2^14 10 (616; 8: 642, 12: 648), 2^16 12-13 (845-850; 10:
+// 897, 14: 996), 2^18 13 (1706; 12: 1734, 15: 1785); BN254 G2 2^16 13 (2387;
+// 10: 2512), BLS12-381 2^16 12 (1524; 13: 1560).
 inline uint32_t choose_window(uint64_t entries_per_window, uint32_t bits) {
     double best = 1e300;
     uint32_t bc = 8;
     for (uint32_t c = 4; c <= 22; c++) {
-        uint32_t w = windows_for(bits, c);
-        double add = (double)entries_per_window * w;
-        double red = 4.2 * (double)w * (double)(1u << (c - 1));
-        double lat = 2.0e5 * (c + 6) + 4.0e4 * (double)w * c;  // serial tails, in madd units
-        double cost = add + red + lat;
+        const double w = windows_for(bits, c), e = (double)entries_per_window * w;
+        const double buckets = w * (double)(1u << (c - 1));
+        double cost = e * (1.0 + 1e6 / (1e6 + e)) + 4.2 * buckets + 5.0e4 * c;
+        if (buckets > RED_QUAD_MAX_NODES) cost += 8.0e5;
         if (cost < best) {
             best = cost;
             bc = c;
@@ -844,14 +851,15 @@ class Engine {
             // long enough to hold about two average buckets and at least 192
             // entries (so few buckets are cut and the partial-sum levels stay
             // small: at 2^24 with ~24 entries per bucket, chunks of 192 beat
-            // chunks of 48 by 0.9 ms), short enough to give at least 8 waves
-            // of resident threads
+            // chunks of 48 by 0.9 ms), short enough to give about 4 waves of
+            // resident threads (each chunk costs two leaves of the next
+            // level: BN254 2^20 4271 us with 8 waves, 4120 with 3.5)
             // (a hint within 10% of the bound is the bound: dense scalar sets
             // keep the plan they get without a sample)
             const uint64_t Me = entries_hint && entries_hint < M - M / 10 ? entries_hint : M;
-            uint64_t waves8 = Me / (8ull * 148 * 512);
+            uint64_t waves4 = Me / (4ull * 148 * 512);
             uint64_t avg = pl.nbuckets ? Me / pl.nbuckets : 1;
-            uint64_t k = std::min<uint64_t>(std::max<uint64_t>(8, waves8), std::max<uint64_t>(192, 2 * avg));
+            uint64_t k = std::min<uint64_t>(std::max<uint64_t>(8, waves4), std::max<uint64_t>(192, 2 * avg));
             K1 = (uint32_t)std::min<uint64_t>(k, 512);
             // then round the thread count to a whole number of waves of
             // resident threads: a last, nearly empty wave would run on an

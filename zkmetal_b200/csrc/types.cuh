@@ -90,10 +90,12 @@ constexpr uint32_t PROFILE_SAMPLES = 4096;
 
 // Segmented sums of the sorted entries (k_acc_fold): leaves per block are
 // FOLD_QUADS * J, J leaves per quad; entry sets up to ACC_FOLD_MAX_ENTRIES
-// skip the one-thread-per-chunk first level.
+// skip the one-thread-per-chunk first level (BN254 1000 points, 64k entries:
+// 457 us either way; 4096 points, 131k entries: 550 us folded, 500 us with
+// chunks of 8 entries first).
 constexpr uint32_t FOLD_THREADS = 256;
 constexpr uint32_t FOLD_QUADS = FOLD_THREADS / 4;
-constexpr uint64_t ACC_FOLD_MAX_ENTRIES = 1ull << 18;
+constexpr uint64_t ACC_FOLD_MAX_ENTRIES = 1ull << 16;
 
 // Bucket reduction: one-thread-per-node levels (k_reduce_level) run while
 // there are more than RED_QUAD_MAX_NODES nodes in all or RED_QUAD_MAX_WINDOW
