@@ -75,11 +75,8 @@ ZK_DEV void fe_sub(Fe<Fp2Of<B>>& r, const Fe<Fp2Of<B>>& a, const Fe<Fp2Of<B>>& b
 }
 
 // (a0 + a1 u)(b0 + b1 u) = (a0 b0 - a1 b1) + ((a0 + a1)(b0 + b1) - a0 b0 - a1 b1) u
-// The base products are always the shared out-of-line copy, also where the
-// caller asks for inline products (INL): three inline 8-limb products per
-// Fp2 product made the G2 kernels too large to compile in reasonable time.
-template <bool INL, class B>
-ZK_DEV void fe_mul_x(Fe<Fp2Of<B>>& r, const Fe<Fp2Of<B>>& a, const Fe<Fp2Of<B>>& b) {
+template <class B>
+ZK_DEV void fe_mul(Fe<Fp2Of<B>>& r, const Fe<Fp2Of<B>>& a, const Fe<Fp2Of<B>>& b) {
     Fe<B> a0, a1, b0, b1, t0, t1, s, t;
     fp2_split(a, a0, a1);
     fp2_split(b, b0, b1);
@@ -92,11 +89,6 @@ ZK_DEV void fe_mul_x(Fe<Fp2Of<B>>& r, const Fe<Fp2Of<B>>& a, const Fe<Fp2Of<B>>&
     fe_sub(s, s, t0);
     fe_sub(a1, s, t1);
     fp2_join(r, a0, a1);
-}
-
-template <class B>
-ZK_DEV void fe_mul(Fe<Fp2Of<B>>& r, const Fe<Fp2Of<B>>& a, const Fe<Fp2Of<B>>& b) {
-    fe_mul_x<false>(r, a, b);
 }
 
 // (a0 + a1 u)^2 = (a0 + a1)(a0 - a1) + 2 a0 a1 u

@@ -1357,9 +1357,9 @@ __global__ void __launch_bounds__(32 * RED_SLOTS1) k_reduce_windows(const Xyzz<t
 // 127), a few additions and one inversion, whatever n is.  A quad (quad.cuh)
 // runs a doubling in two product layers, so the chain is about 250 product
 // times.  Four warps (32 quads) have a scheduler each; more would queue for
-// the multiply pipe, hence the split.  With the bit sums' Horner steps 266 us
-// at 2^8 points (BN254, 32 windows) and 262 us at 2^16 (11 windows), BLS12-377
-// 10^5 487 us, BN254 G2 2^16 844 us; four warps sharing the layers of XYZZ
+// the multiply pipe, hence the split.  With the bit sums' Horner steps 200 us
+// at 2^8 points (BN254, 32 windows) and 196 us at 2^16 (10 windows), BLS12-377
+// 10^5 382 us, BN254 G2 2^16 845 us; four warps sharing the layers of XYZZ
 // doublings through shared memory, with a binary Euclid and without those
 // steps, took 378, 434, 885 and 1034 us.
 struct CombineTerms {
