@@ -239,6 +239,8 @@ struct Tuning {
     // threads of the level-1 accumulation kernel resident at once on the
     // device, per curve (0: unknown; then chunks are not wave-aligned)
     uint32_t acc_wave[NCURVES] = {};
+    // resident blocks of k_acc_fold, per curve (0: unknown)
+    uint32_t fold_blocks[NCURVES] = {};
     // SMs of the device (the MSD sort's first pass runs one group per SM)
     uint32_t sms = 148;
 };
@@ -644,6 +646,10 @@ class Engine {
         tuning.acc_wave[1] = acc_resident_threads<Bls381>();
         tuning.acc_wave[2] = acc_resident_threads<Bls377>();
         tuning.acc_wave[3] = acc_resident_threads<Bn254G2>();
+        tuning.fold_blocks[0] = fold_resident_blocks<Bn254>();
+        tuning.fold_blocks[1] = fold_resident_blocks<Bls381>();
+        tuning.fold_blocks[2] = fold_resident_blocks<Bls377>();
+        tuning.fold_blocks[3] = fold_resident_blocks<Bn254G2>();
     }
     // Second stream and events for host-to-device copies that overlap the
     // compute stream (striped MSMs from host buffers).
@@ -873,9 +879,18 @@ class Engine {
             if (sc.chunk_pct > 0)
                 K1 = (uint32_t)std::min<uint64_t>(4096, std::max<uint64_t>(8, (uint64_t)K1 * sc.chunk_pct / 100));
         }
-        // fold levels: few leaves per quad while a level is latency-bound,
-        // more when its blocks fill the device several times over
-        auto fold_chunk = [](uint64_t m) { return FOLD_QUADS * (m <= (1ull << 18) ? 4u : 16u); };
+        // fold levels: four leaves per quad while a level fits the device at
+        // once (it is latency-bound), else whole waves of blocks with at most
+        // FOLD_MAX_J leaves per quad (BN254 2^20, 610082 leaves, 296 resident
+        // blocks: 596 blocks of J = 16 need a third wave, 530 of J = 18 two;
+        // 4119 and 4057 us for the whole call; BLS12-377 10^5 1781 and 1751)
+        const uint64_t fb = tuning.fold_blocks[CurveTraits<C>::id] ? tuning.fold_blocks[CurveTraits<C>::id] : 296;
+        auto fold_chunk = [fb](uint64_t m) {
+            const uint64_t wave = FOLD_QUADS * fb;  // quads resident
+            const uint64_t waves = (m + wave * FOLD_MAX_J - 1) / (wave * FOLD_MAX_J);
+            const uint64_t J = (m + wave * waves - 1) / (wave * std::max<uint64_t>(waves, 1));
+            return FOLD_QUADS * (uint32_t)std::max<uint64_t>(4, (J + 1) / 2 * 2);
+        };
         pl.acc_fold = tuning.chunk <= 0 && M <= ACC_FOLD_MAX_ENTRIES;
         uint32_t K = pl.acc_fold ? fold_chunk(M) : K1;
         for (int lvl = 0; lvl < 40; lvl++) {
@@ -1126,6 +1141,9 @@ class Engine {
     // resident threads of k_acc_l1<C> on this device (occupancy API)
     template <class C>
     uint32_t acc_resident_threads();
+    // resident blocks of k_acc_fold<C>
+    template <class C>
+    uint32_t fold_resident_blocks();
     template <class C>
     void gen_bases(uint64_t seed, uint64_t index0, uint64_t n, uint32_t* d_out);
     // Histogram of the prepared half lengths of PROFILE_SAMPLES scalars of
@@ -1244,6 +1262,7 @@ class Engine {
     EXT template void Engine::make_phi<C>(const uint32_t*, uint64_t, uint32_t*);                        \
     EXT template void Engine::make_shifts<C>(uint32_t*, uint64_t, uint32_t, uint32_t);                  \
     EXT template uint32_t Engine::acc_resident_threads<C>();                                              \
+    EXT template uint32_t Engine::fold_resident_blocks<C>();                                              \
     EXT template void Engine::gen_bases<C>(uint64_t, uint64_t, uint64_t, uint32_t*);                    \
     EXT template void Engine::profile_scalars<C>(const uint32_t*, uint64_t, int, bool);                 \
     EXT template void Engine::gen_scalars<C>(uint64_t, uint64_t, uint64_t, int, int, uint32_t*);

@@ -312,6 +312,17 @@ uint32_t Engine::acc_resident_threads() {
 }
 
 template <class C>
+uint32_t Engine::fold_resident_blocks() {
+    int per_sm = 0, sms = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_acc_fold<C, false>, FOLD_THREADS, 0) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return (uint32_t)(per_sm * sms);
+}
+
+template <class C>
 void Engine::gen_bases(uint64_t seed, uint64_t index0, uint64_t n, uint32_t* d_out) {
     using P = typename C::Fp;
     const int ci = CurveTraits<C>::id;

@@ -95,6 +95,7 @@ constexpr uint32_t PROFILE_SAMPLES = 4096;
 // chunks of 8 entries first).
 constexpr uint32_t FOLD_THREADS = 256;
 constexpr uint32_t FOLD_QUADS = FOLD_THREADS / 4;
+constexpr uint32_t FOLD_MAX_J = 24;
 constexpr uint64_t ACC_FOLD_MAX_ENTRIES = 1ull << 16;
 
 // Bucket reduction: one-thread-per-node levels (k_reduce_level) run while
