@@ -857,20 +857,24 @@ class Engine {
             // long enough to hold about two average buckets and at least 192
             // entries (so few buckets are cut and the partial-sum levels stay
             // small: at 2^24 with ~24 entries per bucket, chunks of 192 beat
-            // chunks of 48 by 0.9 ms), short enough to give about 4 waves of
-            // resident threads (each chunk costs two leaves of the next
-            // level: BN254 2^20 4271 us with 8 waves, 4120 with 3.5)
+            // chunks of 48 by 0.9 ms), short enough to give two waves of
+            // resident threads, or one where that leaves at most 96 entries
+            // per thread: each chunk costs two leaves of the next level
+            // (BN254 2^20: 56 entries, four waves, 4049 us; 111, two, 4025;
+            // 224, one, 4177; 2^18: 17, four, 1733; 36, two, 1633; 70, one,
+            // 1596; 2^16: 9, two, 783; 18, one, 749)
             // (a hint within 10% of the bound is the bound: dense scalar sets
             // keep the plan they get without a sample)
             const uint64_t Me = entries_hint && entries_hint < M - M / 10 ? entries_hint : M;
-            uint64_t waves4 = Me / (4ull * 148 * 512);
+            const uint64_t W = tuning.acc_wave[CurveTraits<C>::id];
+            const uint64_t R = W ? W : 148ull * 512;
+            uint64_t waves2 = Me <= 96 * R ? Me / R : Me / (2 * R);
             uint64_t avg = pl.nbuckets ? Me / pl.nbuckets : 1;
-            uint64_t k = std::min<uint64_t>(std::max<uint64_t>(8, waves4), std::max<uint64_t>(192, 2 * avg));
+            uint64_t k = std::min<uint64_t>(std::max<uint64_t>(8, waves2), std::max<uint64_t>(192, 2 * avg));
             K1 = (uint32_t)std::min<uint64_t>(k, 512);
             // then round the thread count to a whole number of waves of
             // resident threads: a last, nearly empty wave would run on an
             // almost idle device for a full chunk time
-            const uint64_t W = tuning.acc_wave[CurveTraits<C>::id];
             if (W) {
                 const double waves = (double)Me / ((double)K1 * (double)W);
                 const uint64_t w = (uint64_t)(waves + 0.5);
