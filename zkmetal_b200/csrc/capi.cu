@@ -1033,7 +1033,8 @@ static ZkMetalStatus plan_json(int curve, const uint32_t* counts, uint32_t n_msm
         for (size_t l = 0; l < pl.acc_K.size(); l++)
             s += (l ? "," : "") + std::string("[") + std::to_string(pl.acc_K[l]) + "," + std::to_string(pl.acc_T[l]) +
                  "," + std::to_string(pl.acc_Mbound[l]) + "]";
-        s += "],\"red_L\":" + std::to_string(pl.red_L) + ",\"red_log2L\":" + std::to_string(pl.red_log2L) +
+        s += "],\"affine\":[" + std::to_string(pl.aff_levels) + "," + std::to_string(pl.aff_threads) + "," +
+             std::to_string(pl.aff_slabs) + "],\"red_L\":" + std::to_string(pl.red_L) + ",\"red_log2L\":" + std::to_string(pl.red_log2L) +
              ",\"red\":[";
         for (size_t l = 0; l < pl.red_tasks.size(); l++) {
             s += (l ? "," : "") + std::string("[");

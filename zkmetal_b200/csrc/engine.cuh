@@ -241,6 +241,8 @@ struct Tuning {
     uint32_t acc_wave[NCURVES] = {};
     // resident blocks of k_acc_fold, per curve (0: unknown)
     uint32_t fold_blocks[NCURVES] = {};
+    // the same for the affine sums (threads per slab)
+    uint32_t aff_wave[NCURVES] = {};
     // SMs of the device (the MSD sort's first pass runs one group per SM)
     uint32_t sms = 148;
 };
@@ -266,6 +268,10 @@ struct Plan {
     // segmented-sum levels: chunk length and chunk-count bound per level;
     // acc_fold: the first level runs k_acc_fold too (else k_acc_l1)
     bool acc_fold = false;
+    // levels of affine pair sums before the chunks' XYZZ sums (0: none), the
+    // threads (chunks) of a slab, and the slabs the expected entries fill
+    // (chunks past them, if there are more entries, take k_acc_l1)
+    uint32_t aff_levels = 0, aff_threads = 0, aff_slabs = 0;
     std::vector<uint32_t> acc_K, acc_T;
     std::vector<uint64_t> acc_Mbound;
     // bucket-reduction tree (levels of arity red_L to one node per window); the
@@ -301,6 +307,7 @@ struct Plan {
         red_log2L = 3;
         acc_threads = 0;
         acc_fold = false;
+        aff_levels = aff_threads = aff_slabs = 0;
         acc_K.clear();
         acc_T.clear();
         acc_Mbound.clear();
@@ -321,6 +328,36 @@ inline uint64_t msd_rows_words(const Plan& pl) {
 inline uint64_t msd_scan_words(const Plan& pl) {
     return std::max<uint64_t>((uint64_t)(1u << pl.msd_bits1) * pl.msd_groups1 * MSD_COUNT_PARTS,
                               pl.msd_passes == 2 ? (uint64_t)(1u << pl.msd_bits2) * pl.msd_chunks2 : 0);
+}
+
+// Byte offsets of the affine slab's buffers (AffSlab in affine.cuh): 62 bytes
+// per entry of a slab's chunks and a few dozen per thread at 8 limbs.
+struct AffLayout {
+    uint32_t pcap = 0;
+    size_t pts = 0, pre = 0, info = 0, elem = 0, runs = 0, prod = 0, cnt = 0, npair = 0, bytes = 0;
+};
+template <class P>
+inline AffLayout aff_layout(const Plan& pl) {
+    AffLayout a;
+    if (!pl.aff_levels) return a;
+    const size_t K = pl.acc_K[0], T = pl.aff_threads, fb = P::N * 4;
+    a.pcap = (uint32_t)(K / 2);
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        const size_t o = off;
+        off = (off + bytes + 255) / 256 * 256;
+        return o;
+    };
+    a.pts = take(T * a.pcap * 2 * fb);
+    a.pre = take(T * a.pcap * fb);
+    a.info = take(T * a.pcap * 8);
+    a.elem = take(T * K * 2);
+    a.runs = take(T * K * 8);
+    a.prod = take(T * fb);
+    a.cnt = take(T * 4);
+    a.npair = take(T * 4);
+    a.bytes = off;
+    return a;
 }
 
 // Nearest power-of-two exponent of n (n >= 1).
@@ -553,6 +590,8 @@ struct CurveTraits<Bn254G2> {
     static constexpr uint32_t fr_bits = Bn254Fr::BITS;
 };
 
+struct AffSlab;  // affine.cuh
+
 class Engine {
    public:
     cudaStream_t stream = nullptr;
@@ -609,7 +648,7 @@ class Engine {
     DevBuf w_points, w_phi, w_scalars, w_ents, w_buckets;
     DevBuf w_ents2, w_thist, w_stripe_buckets, w_seg;
     DevBuf w_tiles, w_totals, w_pkeys[2], w_pvals[2], w_redS[2], w_redW[2];
-    DevBuf w_quad1, w_quad2, w_results, w_comb, w_profile;
+    DevBuf w_aff, w_quad1, w_quad2, w_results, w_comb, w_profile;
     uint32_t* h_profile = nullptr;  // pinned, PROFILE_BINS words
     bool comb_ready[NCURVES] = {};
     uint32_t* h_results = nullptr;  // pinned
@@ -622,7 +661,7 @@ class Engine {
         DevBuf* bufs[] = {&w_points, &w_phi, &w_scalars, &w_ents, &w_buckets,
                           &w_ents2, &w_thist, &w_stripe_buckets, &w_seg, &w_tiles, &w_totals,
                           &w_pkeys[0], &w_pkeys[1], &w_pvals[0], &w_pvals[1], &w_redS[0], &w_redS[1],
-                          &w_redW[0], &w_redW[1], &w_quad1, &w_quad2, &w_results, &w_comb, &w_profile, &transient.d_descs,
+                          &w_redW[0], &w_redW[1], &w_aff, &w_quad1, &w_quad2, &w_results, &w_comb, &w_profile, &transient.d_descs,
                           &transient.d_tasks};
         for (DevBuf* b : bufs) b->sp = &stream;
         cudaMemPool_t pool;
@@ -650,6 +689,10 @@ class Engine {
         tuning.fold_blocks[1] = fold_resident_blocks<Bls381>();
         tuning.fold_blocks[2] = fold_resident_blocks<Bls377>();
         tuning.fold_blocks[3] = fold_resident_blocks<Bn254G2>();
+        tuning.aff_wave[0] = aff_resident_threads<Bn254>();
+        tuning.aff_wave[1] = aff_resident_threads<Bls381>();
+        tuning.aff_wave[2] = aff_resident_threads<Bls377>();
+        tuning.aff_wave[3] = aff_resident_threads<Bn254G2>();
     }
     // Second stream and events for host-to-device copies that overlap the
     // compute stream (striped MSMs from host buffers).
@@ -883,6 +926,27 @@ class Engine {
             if (sc.chunk_pct > 0)
                 K1 = (uint32_t)std::min<uint64_t>(4096, std::max<uint64_t>(8, (uint64_t)K1 * sc.chunk_pct / 100));
         }
+        // affine pair sums: runs of at least AFF_MIN_RUN on average.  One wave
+        // of threads per slab, chunks of at most AFF_MAX_CHUNK entries; a
+        // level for each halving of the average run, while a thread has
+        // several pairs to share an inversion's cost
+        {
+            const uint64_t Me = entries_hint && entries_hint < M - M / 10 ? entries_hint : M;
+            const uint64_t run = Me / std::max<uint32_t>(pl.nbuckets, 1);
+            if (AFF_CURVE<C> && tuning.chunk <= 0 && Me >= AFF_MIN_ENTRIES && run >= AFF_MIN_RUN) {
+                uint32_t W = tuning.aff_wave[CurveTraits<C>::id];
+                W = std::max(AFF_SLAB_UNIT, (W ? W : AFF_SLAB_DEFAULT) / AFF_SLAB_UNIT * AFF_SLAB_UNIT);
+                const uint64_t slabs = (Me + (uint64_t)W * AFF_MAX_CHUNK - 1) / ((uint64_t)W * AFF_MAX_CHUNK);
+                K1 = (uint32_t)((Me + slabs * W - 1) / (slabs * W));
+                if (sc.chunk_pct > 0) K1 = std::min<uint32_t>(2 * AFF_MAX_CHUNK, K1 * sc.chunk_pct / 100);
+                K1 = std::max<uint32_t>((K1 + 3) / 4 * 4, 16);
+                pl.aff_threads = W;
+                pl.aff_slabs = (uint32_t)slabs;
+                while (pl.aff_levels < 8 && (K1 >> (pl.aff_levels + 1)) >= 4 &&
+                       2 * run >= (3ull << pl.aff_levels))  // 1.5 per run left to halve
+                    pl.aff_levels++;
+            }
+        }
         // fold levels: four leaves per quad while a level fits the device at
         // once (it is latency-bound), else whole waves of blocks with at most
         // FOLD_MAX_J leaves per quad (BN254 2^20, 610082 leaves, 296 resident
@@ -1071,6 +1135,7 @@ class Engine {
         uint64_t m2 = 2, m3 = 2;
         if (pl.acc_Mbound.size() > 1) m2 = pl.acc_Mbound[1];
         for (size_t l = 2; l < pl.acc_Mbound.size(); l++) m3 = std::max<uint64_t>(m3, pl.acc_Mbound[l]);
+        if (pl.aff_levels) grew |= w_aff.ensure(aff_layout<P>(pl).bytes);
         grew |= w_pkeys[0].ensure(m2 * 4 + 16);
         grew |= w_pvals[0].ensure(m2 * xs + xs);
         grew |= w_pkeys[1].ensure(m3 * 4 + 16);
@@ -1148,6 +1213,11 @@ class Engine {
     // resident blocks of k_acc_fold<C>
     template <class C>
     uint32_t fold_resident_blocks();
+    // the same of k_aff_add<C>, in whole blocks of every affine kernel
+    template <class C>
+    uint32_t aff_resident_threads();
+    template <class C>
+    AffSlab aff_slab(const Plan& pl) const;
     template <class C>
     void gen_bases(uint64_t seed, uint64_t index0, uint64_t n, uint32_t* d_out);
     // Histogram of the prepared half lengths of PROFILE_SAMPLES scalars of
@@ -1267,6 +1337,7 @@ class Engine {
     EXT template void Engine::make_shifts<C>(uint32_t*, uint64_t, uint32_t, uint32_t);                  \
     EXT template uint32_t Engine::acc_resident_threads<C>();                                              \
     EXT template uint32_t Engine::fold_resident_blocks<C>();                                              \
+    EXT template uint32_t Engine::aff_resident_threads<C>();                                              \
     EXT template void Engine::gen_bases<C>(uint64_t, uint64_t, uint64_t, uint32_t*);                    \
     EXT template void Engine::profile_scalars<C>(const uint32_t*, uint64_t, int, bool);                 \
     EXT template void Engine::gen_scalars<C>(uint64_t, uint64_t, uint64_t, int, int, uint32_t*);

@@ -2,6 +2,7 @@
 // by the per-curve instantiation units so each curve's kernels compile once.
 #pragma once
 #include "engine.cuh"
+#include "affine.cuh"
 #include "msm_kernels.cuh"
 
 #include <mutex>
@@ -9,6 +10,8 @@
 #include <utility>
 
 namespace zkmsm {
+
+static_assert(AFF_SLAB_UNIT % (AFF_THREADS * AFF_G) == 0, "a slab is whole blocks of every affine kernel");
 
 // Exclusive scan of n u32 in place; total to d_total; optional copy.
 static void scan_u32(Engine& e, uint32_t* d_in_out, uint32_t n, uint32_t* d_total, uint32_t* d_copy) {
@@ -178,12 +181,44 @@ void Engine::enqueue(const Plan& pl, const uint32_t* d_bases, const uint32_t* d_
         uint32_t* d_next = tot + l + 1;
         uint32_t* okeys = w_pkeys[cur].as<uint32_t>();
         Xyzz<P>* ovals = w_pvals[cur].as<Xyzz<P>>();
-        if (l == 0 && !pl.acc_fold) {
+        // k_acc_l1 over chunks [t0, T)
+        auto level1 = [&](uint32_t t0) {
             const uint32_t AT = pl.acc_threads && pl.acc_threads <= (uint32_t)AccLaunch<C>::THREADS
                                         ? pl.acc_threads
                                         : (uint32_t)AccLaunch<C>::THREADS;
-            k_acc_l1<C><<<(T + AT - 1) / AT, AT, 0, stream>>>(w_ents.as<uint2>(), d_len, K, d_bases, d_phi, d_next,
-                                                             buckets, okeys, ovals);
+            k_acc_l1<C><<<(T - t0 + AT - 1) / AT, AT, 0, stream>>>(w_ents.as<uint2>(), d_len, K, t0, d_bases, d_phi,
+                                                                  d_next, buckets, okeys, ovals);
+        };
+        if (l == 0 && pl.aff_levels) {
+          if constexpr (AFF_CURVE<C>) {
+            const AffSlab sl = aff_slab<C>(pl);
+            const uint32_t nb = sl.threads / AFF_THREADS;
+            const uint64_t end = (uint64_t)pl.aff_slabs * sl.threads;
+            for (uint64_t g0 = 0; g0 < end; g0 += sl.threads) {
+                for (uint32_t a = 0; a < pl.aff_levels; a++) {
+                    const uint2* ents = w_ents.as<uint2>();
+                    if (a == 0)
+                        k_aff_pair<C, true><<<nb, AFF_THREADS, 0, stream>>>(sl, ents, d_len, g0, d_bases, d_phi);
+                    else
+                        k_aff_pair<C, false><<<nb, AFF_THREADS, 0, stream>>>(sl, ents, d_len, g0, d_bases, d_phi);
+                    k_aff_invert<C><<<nb / AFF_G, AFF_THREADS, 0, stream>>>(sl.prod, sl.threads);
+                    if (a == 0) k_aff_add<C, true><<<nb, AFF_THREADS, 0, stream>>>(sl, d_bases, d_phi);
+                    else k_aff_add<C, false><<<nb, AFF_THREADS, 0, stream>>>(sl, d_bases, d_phi);
+                    launches += 3;
+                    ZK_CUDA(cudaGetLastError());
+                }
+                k_aff_finish<C><<<nb, AFF_THREADS, 0, stream>>>(sl, d_len, g0, d_bases, d_phi, d_next, buckets, okeys,
+                                                                ovals);
+                if (g0 + sl.threads < end) launches++;  // the last launch is counted below
+                ZK_CUDA(cudaGetLastError());
+            }
+            if (end < T) {
+                launches++;
+                level1((uint32_t)end);
+            }
+          }
+        } else if (l == 0 && !pl.acc_fold) {
+            level1(0);
         } else if (l == 0) {
             k_acc_fold<C, true><<<T, FOLD_THREADS, 0, stream>>>(w_ents.as<uint2>(), d_bases, d_phi, nullptr, nullptr,
                                                                 d_len, K / FOLD_QUADS, last, d_next, buckets, okeys,
@@ -201,6 +236,26 @@ void Engine::enqueue(const Plan& pl, const uint32_t* d_bases, const uint32_t* d_
     prof_mark(ev, 3);
     if (!(flags & ENQ_ACC_ONLY)) enqueue_reduce<C>(pl, buckets, d_results, &ev);
     prof_end(ev);
+}
+
+// The buffers of an affine slab inside w_aff (sized by aff_slab_bytes).
+template <class C>
+AffSlab Engine::aff_slab(const Plan& pl) const {
+    const AffLayout a = aff_layout<typename C::Fp>(pl);
+    uint8_t* b = w_aff.as<uint8_t>();
+    AffSlab s;
+    s.pts = reinterpret_cast<uint4*>(b + a.pts);
+    s.pre = reinterpret_cast<uint4*>(b + a.pre);
+    s.info = reinterpret_cast<uint2*>(b + a.info);
+    s.elem = reinterpret_cast<uint2*>(b + a.elem);
+    s.runs = reinterpret_cast<uint2*>(b + a.runs);
+    s.prod = reinterpret_cast<uint32_t*>(b + a.prod);
+    s.cnt = reinterpret_cast<uint32_t*>(b + a.cnt);
+    s.npair = reinterpret_cast<uint32_t*>(b + a.npair);
+    s.K = pl.acc_K[0];
+    s.pcap = a.pcap;
+    s.threads = pl.aff_threads;
+    return s;
 }
 
 // Window sums from the buckets (running sums, then bit sums by quads), then
@@ -320,6 +375,20 @@ uint32_t Engine::fold_resident_blocks() {
         return 0;
     }
     return (uint32_t)(per_sm * sms);
+}
+
+template <class C>
+uint32_t Engine::aff_resident_threads() {
+    if constexpr (!AFF_CURVE<C>) return 0;
+    else {
+    int per_sm = 0, sms = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_aff_add<C, false>, AFF_THREADS, 0) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return (uint32_t)(per_sm * sms) * AFF_THREADS;
+    }
 }
 
 template <class C>

@@ -912,7 +912,7 @@ struct AccLaunch<Bls377> {  // the same 12-limb arithmetic as BLS12-381
 };
 template <class C>
 __global__ void __launch_bounds__(AccLaunch<C>::THREADS, AccLaunch<C>::MIN_BLOCKS) k_acc_l1(const uint2* __restrict__ ents,
-                                                const uint32_t* __restrict__ d_len, uint32_t K,
+                                                const uint32_t* __restrict__ d_len, uint32_t K, uint32_t t0,
                                                 const uint32_t* __restrict__ bases,
                                                 const uint32_t* __restrict__ phi,
                                                 uint32_t* __restrict__ d_next,
@@ -920,7 +920,7 @@ __global__ void __launch_bounds__(AccLaunch<C>::THREADS, AccLaunch<C>::MIN_BLOCK
                                                 uint32_t* __restrict__ pkeys,
                                                 Xyzz<typename C::Fp>* __restrict__ pvals) {
     using P = typename C::Fp;
-    uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t t = t0 + blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t M = *d_len;
     if (t == 0) *d_next = (uint32_t)(2 * (((uint64_t)M + K - 1) / K));
     uint64_t start64 = (uint64_t)t * K;

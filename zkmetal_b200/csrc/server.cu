@@ -466,13 +466,19 @@ ZkMetalStatus zkmsm_server_create(ZkMsmTable bn254_table, ZkMsmTable bls12_381_t
     // milliseconds.  Memory reserved once and kept by the pool is handed out
     // without mapping.  A worker's workspace for a full batch of small and
     // medium MSMs over window-shift tables (one sorted entry per window per
-    // point, two entry arrays, scalars) reaches about 480 B per batch point.
+    // point, two entry arrays, scalars) reaches about 480 B per batch point;
+    // BLS12-381 batches add a slab of affine sums, 86 B for each of at most
+    // 13 entries per point and one wave of the longest chunks.
     {
         size_t fr = 0, tot = 0;
         cudaMemPool_t pool;
         if (cudaMemGetInfo(&fr, &tot) == cudaSuccess && cudaDeviceGetDefaultMemPool(&pool, s->device) == cudaSuccess) {
+            const uint64_t slab =
+                    bls12_381_table
+                            ? std::min<uint64_t>(s->max_batch_points * 13, (uint64_t)AFF_SLAB_DEFAULT * AFF_MAX_CHUNK) * 86
+                            : 0;
             const uint64_t want =
-                    std::min<uint64_t>((uint64_t)workers * s->max_batch_points * 512 + (1ull << 30), fr / 4);
+                    std::min<uint64_t>((uint64_t)workers * (s->max_batch_points * 512 + slab) + (1ull << 30), fr / 4);
             uint64_t thr = 0;
             cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
             if (thr < want) {

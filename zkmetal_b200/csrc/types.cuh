@@ -98,6 +98,23 @@ constexpr uint32_t FOLD_QUADS = FOLD_THREADS / 4;
 constexpr uint32_t FOLD_MAX_J = 24;
 constexpr uint64_t ACC_FOLD_MAX_ENTRIES = 1ull << 16;
 
+// Affine accumulation (affine.cuh): the curves that take it, the smallest
+// entry set and mean run length, the longest chunk, threads per slab unit, and
+// the slab used where the device is not known (plans described without a GPU).
+// Four products saved per addition are worth the second fetch of its points
+// where a product is long: BLS12-381 2^20 7403 us against 7859 in chunks of
+// k_acc_l1, 2^22 24.5 and 25.8 ms, BLS12-377 2^18 2808 and 3022 us, BN254 G2
+// 2^18 4358 and 4691 us, 2^20 10.8 and 12.1 ms; BN254 G1 2^20 4277 and 4025
+// us, 2^24 49.4 and 44.2 ms (there the random fetches from 2 GB of points,
+// 39 G sectors/s, take as long as the products).
+template <class C>
+constexpr bool AFF_CURVE = C::Fp::N >= 12;
+constexpr uint64_t AFF_MIN_ENTRIES = 1ull << 22;
+constexpr uint64_t AFF_MIN_RUN = 8;
+constexpr uint32_t AFF_MAX_CHUNK = 512;
+constexpr uint32_t AFF_SLAB_UNIT = 512;
+constexpr uint32_t AFF_SLAB_DEFAULT = 148 * 512;
+
 // Bucket reduction: one-thread-per-node levels (k_reduce_level) run while
 // there are more than RED_QUAD_MAX_NODES nodes in all or RED_QUAD_MAX_WINDOW
 // in a window; k_reduce_quads takes the rest, one node per quad while the
