@@ -284,7 +284,12 @@ void Engine::enqueue_reduce(const Plan& pl, const void* bucket_base, uint32_t* d
     }
     const RedTask* qt = pl.d_tasks.as<RedTask>() + pl.task_level_off.back();
     const uint32_t nw = (uint32_t)pl.quad_tasks.size(), span = pl.red_levels * pl.red_log2L;
-    CombineTerms ct{RED_SLOTS1, span + pl.quad_log2J, 0, 0};
+    // T_j of quads no window reaches are zero: small windows have few terms
+    uint32_t quads = 1, tb = 0;
+    for (const auto& t : pl.quad_tasks)
+        quads = std::max(quads, std::min(RED_QUADS, (t.n_in + (1u << pl.quad_log2J) - 1) >> pl.quad_log2J));
+    while ((1u << tb) < quads) tb++;
+    CombineTerms ct{RED_SLOTS1, 2 + tb, span + pl.quad_log2J, 0, 0};
     Xyzz<P>* terms = w_quad1.as<Xyzz<P>>();
     if (pl.quad_blocks) {
         k_reduce_quads<C><<<pl.quad_blocks, 4 * RED_QUADS, 0, stream>>>(inS, inW, qt, (int)nw, 1u << pl.quad_log2J, span,
@@ -297,7 +302,7 @@ void Engine::enqueue_reduce(const Plan& pl, const void* bucket_base, uint32_t* d
         launches++;
         ZK_CUDA(cudaGetLastError());
         terms = w_quad2.as<Xyzz<P>>();
-        ct.slots = RED_SLOTS2;
+        ct.slots = ct.used = RED_SLOTS2;
         ct.bit_x = ct.bit_t + 6;  // log2(RED_QUADS) bits of T
         ct.bit_t2 = ct.bit_x + pl.quad_log2E;
     }

@@ -1364,6 +1364,7 @@ __global__ void __launch_bounds__(32 * RED_SLOTS1) k_reduce_windows(const Xyzz<t
 // steps, took 378, 434, 885 and 1034 us.
 struct CombineTerms {
     uint32_t slots;     // points per window: RED_SLOTS1 or RED_SLOTS2
+    uint32_t used;      // positions (term_slot) that hold points; the rest are zero
     uint32_t bit_t;     // bit of T_0
     uint32_t bit_x;     // RED_SLOTS2: bit of X, and of T'_0
     uint32_t bit_t2;
@@ -1406,14 +1407,15 @@ __global__ void __launch_bounds__(4 * MAX_WINDOWS) k_combine(const Xyzz<typename
         return;
     }
     const uint32_t split = combine_split(d.nred), nq = d.nred * split;  // quads in use
-    const uint32_t w = u / split, per = ct.slots / split;
+    const uint32_t w = u / split, per = (ct.used + split - 1) / split;
     const uint32_t lo = (u % split) * per;  // this quad's terms: positions [lo, lo + per)
-    const bool live = u < nq;
+    // (split divides RED_SLOTS1 and RED_SLOTS2, so positions stay below slots)
+    const bool live = u < nq && lo < ct.used;
     const Xyzz<P>* wt = terms + (size_t)(d.win_off + w) * ct.slots;
     Fe<P> a, b;
     fe_set_zero(a);
     if (8 * warp < nq) {  // warp-uniform
-        if (live) quad_load(a, wt + term_slot(lo + per - 1), q);
+        if (live && lo + per <= ct.used) quad_load(a, wt + term_slot(lo + per - 1), q);
 #pragma unroll 1
         for (uint32_t k = per - 1; k-- > 0;) {
             const uint32_t cnt = live ? term_bit(lo + k + 1, ct) - term_bit(lo + k, ct) : 0u;
@@ -1425,7 +1427,7 @@ __global__ void __launch_bounds__(4 * MAX_WINDOWS) k_combine(const Xyzz<typename
                 fe_select(a, i < cnt, b, a);
             }
             fe_set_zero(b);
-            if (live) quad_load(b, wt + term_slot(lo + k), q);
+            if (live && lo + k < ct.used) quad_load(b, wt + term_slot(lo + k), q);
             quad_add(a, b, q);
         }
         // down to bit 0; a warp runs to the most of its quads
