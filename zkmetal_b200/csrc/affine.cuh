@@ -250,13 +250,16 @@ __global__ void __launch_bounds__(AFF_THREADS, AffLaunch<C>::BLOCKS) k_aff_pair(
     // FIRST: entries i, i + 1, i + 2, fetched ahead of their use
     const uint2 none = make_uint2(ACC_EMPTY, 0);
     uint2 e0 = none, e1 = none, e2 = none;
-    uint32_t sval = 0;  // later levels: the entry kept with the current run
+    // later levels: the entry kept with the current run, and the next run's on
+    // its way
+    uint32_t sval = 0, snext = 0;
     if (FIRST) {
         if (n > 0) e0 = en[0];
         if (n > 1) e1 = en[1];
         if (n > 2) e2 = en[2];
     } else if (n) {
         sval = runs[0].y;
+        snext = runs[32].y;  // K >= 16 rows
     }
     // the next pair of neighbours of one run, its x on their way to slot `at`;
     // what has no partner stays listed
@@ -298,7 +301,10 @@ __global__ void __launch_bounds__(AFF_THREADS, AffLaunch<C>::BLOCKS) k_aff_pair(
                     i += 2;
                     got = true;
                 }
-                if (last & AFF_LAST && i < n) sval = runs[32 * ++run].y;
+                if (last & AFF_LAST) {
+                    sval = snext;
+                    if (++run + 1 < s.K) snext = runs[32 * (run + 1)].y;
+                }
             }
         }
         if (got) {
