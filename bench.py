@@ -117,8 +117,8 @@ def plan_of(n, window=0, curve=0):
 def reduction_products(plan, curve="bn254"):
     """Word products of the bucket reduction's additions: in the levels of the
     plan's tree that k_reduce_level runs, a node of cnt children does
-    2(cnt - 1) + 1 XYZZ additions, cnt more above level 0 (the weighted sums),
-    and level * log2(L) doublings; below them the quads' bit sums take two
+    2 cnt - 3 XYZZ additions (the first of each running sum is a copy), cnt
+    more above level 0 (the weighted sums), and level * log2(L) doublings; below them the quads' bit sums take two
     additions per node."""
     L, lg = plan["red_L"], plan["red_log2L"]
     quad = plan["quad"]
@@ -126,7 +126,7 @@ def reduction_products(plan, curve="bn254"):
     for lvl, tasks in enumerate(plan["red"][:quad["levels"]]):
         for (_, n_in, _, _) in tasks:
             for cnt, k in ((L, n_in // L), (n_in % L, 1 if n_in % L else 0)):
-                adds += (2 * (cnt - 1) + 1 + (cnt if lvl else 0)) * k
+                adds += (max(0, 2 * cnt - 3) + (cnt if lvl else 0)) * k
                 dbls += lvl * lg * k
     return (adds * ADD_MULS + dbls * DBL_MULS) * PRODUCTS_PER_MUL[curve]
 

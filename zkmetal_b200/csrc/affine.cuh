@@ -183,8 +183,8 @@ struct AffList {
     }
 };
 
-// Launch shapes: a slab is the threads of k_aff_add resident at once (8 limbs:
-// five blocks of 128 threads at 102 registers; 12 limbs: four; Fp2: three).
+// Launch shapes: a slab is the threads of k_aff_add resident at once (12 limbs:
+// four blocks of 128 threads, with three the sums are 5% slower; Fp2: three).
 constexpr uint32_t AFF_THREADS = 128;
 template <class C>
 struct AffLaunch {
