@@ -1434,14 +1434,24 @@ __global__ void __launch_bounds__(4 * MAX_WINDOWS) k_combine(const Xyzz<typename
         const uint32_t cnt = live ? win_bit(d, w) + term_bit(lo, ct) : 0u;
         const uint32_t most = __reduce_max_sync(0xffffffffu, cnt);
         if (most) {
-            QuadChain<C>::enter(a, q);
+            const bool chain = QuadChain<C>::on_curve(a, q);
+            if (__all_sync(0xffffffffu, chain)) {
+                QuadChain<C>::enter(a, q);
 #pragma unroll 1
-            for (uint32_t i = 0; i < most; i++) {
-                b = a;
-                QuadChain<C>::dbl(b, q);
-                fe_select(a, i < cnt, b, a);
+                for (uint32_t i = 0; i < most; i++) {
+                    b = a;
+                    QuadChain<C>::dbl(b, q);
+                    fe_select(a, i < cnt, b, a);
+                }
+                QuadChain<C>::leave(a, q);
+            } else {  // points off the curve in this warp
+#pragma unroll 1
+                for (uint32_t i = 0; i < most; i++) {
+                    b = a;
+                    quad_dbl(b, q);
+                    fe_select(a, i < cnt, b, a);
+                }
             }
-            QuadChain<C>::leave(a, q);
         }
     }
     for (uint32_t st = 1; st < nq; st <<= 1) {
