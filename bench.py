@@ -122,7 +122,7 @@ def reduction_products(plan, curve="bn254"):
     additions per node."""
     L, lg = plan["red_L"], plan["red_log2L"]
     quad = plan["quad"]
-    adds, dbls = 2 * sum(t[1] for t in quad["tasks"]), 0
+    adds, dbls = 0 if quad["direct"] else 2 * sum(t[1] for t in quad["tasks"]), 0
     for lvl, tasks in enumerate(plan["red"][:quad["levels"]]):
         for (_, n_in, _, _) in tasks:
             for cnt, k in ((L, n_in // L), (n_in % L, 1 if n_in % L else 0)):

@@ -46,8 +46,12 @@ def reduce_model(pl, buckets):
                     (sum(inW[c] for c in ch) if inW else 0)
         inS, inW = oS, oW
     J, E, span = 1 << Q["log2J"], 1 << Q["log2E"], Q["levels"] * lg
+    assert not (Q["direct"] and (Q["windows"] or any(t[1] != 1 for t in Q["tasks"])))
     out = [[0] * SLOTS1 for _ in range(Q["blocks"])]
     for in_off, n_in, out_off, n_out in Q["tasks"]:
+        # what the block's quads (a power of two, a warp at least) reach
+        assert min(QUADS * J, n_in) <= Q["quads"] * J and Q["quads"] in (8, 16, 32, 64)
+        assert not Q["windows"] or Q["quads"] == QUADS
         assert n_out == -(-n_in // (QUADS * J))
         for b in range(n_out):
             n0 = b * QUADS * J
@@ -102,3 +106,20 @@ def test_quad_reduction_batches():
     check(plan(zl.BLS12_381, [700, 0, 1 << 16, 3]), 1)
     check(plan_shift(zl.BN254, [1, 400, 1 << 17, 9000], 4, 1 << 17), 2)
     check(plan_shift(zl.BN254, [1 << 18], 4, 1 << 18), 3)
+
+
+@pytest.mark.parametrize("counts", [[64] * 256, [16] * 400, [40] * 1024, [1000] * 300, [3000] * 200 + [0, 1 << 17]])
+def test_quad_reduction_many_windows(counts):
+    """Batches of many small MSMs: what the quads' warps add up follows the
+    nodes there are, not 64 quads for each of thousands of windows."""
+    pl = plan(zl.BN254, counts)
+    Q = pl["quad"]
+    nodes = [t[1] for t in Q["tasks"]]
+    if max(nodes) == 1 and Q["levels"]:
+        assert Q["direct"]
+    else:
+        # a block is no wider than the largest window needs
+        assert Q["quads"] == 8 or Q["quads"] << Q["log2J"] < 2 * max(nodes)
+        warps = sum(-(-min(n, 64 << Q["log2J"]) // (8 << Q["log2J"])) for n in nodes)
+        assert 8 * warps <= 2 * (sum(nodes) >> Q["log2J"]) + 8 * len(nodes)
+    check(pl, len(counts))

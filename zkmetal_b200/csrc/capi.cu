@@ -1047,7 +1047,8 @@ static ZkMetalStatus plan_json(int curve, const uint32_t* counts, uint32_t n_msm
         }
         s += "],\"quad\":{\"levels\":" + std::to_string(pl.red_levels) + ",\"log2J\":" +
              std::to_string(pl.quad_log2J) + ",\"log2E\":" + std::to_string(pl.quad_log2E) + ",\"blocks\":" +
-             std::to_string(pl.quad_blocks) + ",\"windows\":" + std::to_string(pl.quad_windows ? 1 : 0) +
+             std::to_string(pl.quad_blocks) + ",\"quads\":" + std::to_string(pl.quad_count) + ",\"direct\":" +
+             std::to_string(pl.red_direct ? 1 : 0) + ",\"windows\":" + std::to_string(pl.quad_windows ? 1 : 0) +
              ",\"tasks\":[";
         for (size_t k = 0; k < pl.quad_tasks.size(); k++) {
             auto& tk = pl.quad_tasks[k];

@@ -278,9 +278,12 @@ struct Plan {
     // first red_levels of them run as kernels, and k_reduce_quads (quad_J =
     // 2^quad_log2J nodes per quad, quad_tasks: one per window) and, when a
     // window has several blocks, k_reduce_windows (2^quad_log2E blocks per
-    // quad) do the work of the rest
-    uint32_t red_levels = 0, quad_log2J = 0, quad_blocks = 0, quad_log2E = 0;
-    bool quad_windows = false;
+    // quad) do the work of the rest, in blocks
+    // of a block's quads (quad_count: as many as the largest window fills).
+    // red_direct: the levels reach one node per window, which is all the
+    // combine needs; no quads run
+    uint32_t red_levels = 0, quad_log2J = 0, quad_blocks = 0, quad_log2E = 0, quad_count = RED_QUADS;
+    bool quad_windows = false, red_direct = false;
     std::vector<RedTask> quad_tasks;
     uint32_t red_L = 8, red_log2L = 3;
     // threads per block of the level-1 accumulation (0: the curve's default)
@@ -301,7 +304,8 @@ struct Plan {
         msd_passes = msd_bits1 = msd_bits2 = msd_tiles1 = msd_tiles2 = 0;
         msd_groups1 = msd_chunks2 = 0;
         red_levels = quad_log2J = quad_blocks = quad_log2E = 0;
-        quad_windows = false;
+        quad_count = RED_QUADS;
+        quad_windows = red_direct = false;
         quad_tasks.clear();
         red_L = 8;
         red_log2L = 3;
@@ -1026,6 +1030,12 @@ class Engine {
             pl.red_levels = lvl;
             if ((total <= RED_QUAD_MAX_NODES && most <= RED_QUAD_MAX_WINDOW) || lvl == pl.red_tasks.size()) {
                 pl.quad_log2J = most <= 8 * RED_QUADS ? 0 : 2;
+                pl.red_direct = lvl > 0 && most == 1;
+                // a block of no more quads than its window has nodes for (a
+                // warp at least): batches of many small MSMs have thousands of
+                // windows of eight nodes
+                pl.quad_count = 8;
+                while (pl.quad_count < RED_QUADS && pl.quad_count << pl.quad_log2J < most) pl.quad_count *= 2;
                 break;
             }
         }

@@ -274,8 +274,14 @@ void Engine::enqueue_reduce(const Plan& pl, const void* bucket_base, uint32_t* d
         const RedTask* tk = pl.d_tasks.as<RedTask>() + pl.task_level_off[l];
         Xyzz<P>* oS = w_redS[rc].as<Xyzz<P>>();
         Xyzz<P>* oW = w_redW[rc].as<Xyzz<P>>();
+        uint32_t step = 1;
+        if (pl.red_direct && l + 1 == pl.red_levels) {  // S and W where the quads' blocks would put them
+            oS = w_quad1.as<Xyzz<P>>();
+            oW = oS + RED_SLOTS1 - 1;
+            step = RED_SLOTS1;
+        }
         k_reduce_level<C><<<(nout + 127) / 128, 128, 0, stream>>>(inS, inW, tk, (int)pl.red_tasks[l].size(), nout,
-                                                                 pl.red_L, (uint32_t)l * pl.red_log2L, oS, oW);
+                                                                 pl.red_L, (uint32_t)l * pl.red_log2L, step, oS, oW);
         launches++;
         ZK_CUDA(cudaGetLastError());
         inS = oS;
@@ -291,9 +297,9 @@ void Engine::enqueue_reduce(const Plan& pl, const void* bucket_base, uint32_t* d
     while ((1u << tb) < quads) tb++;
     CombineTerms ct{RED_SLOTS1, 2 + tb, span + pl.quad_log2J, 0, 0};
     Xyzz<P>* terms = w_quad1.as<Xyzz<P>>();
-    if (pl.quad_blocks) {
-        k_reduce_quads<C><<<pl.quad_blocks, 4 * RED_QUADS, 0, stream>>>(inS, inW, qt, (int)nw, 1u << pl.quad_log2J, span,
-                                                                       terms);
+    if (pl.quad_blocks && !pl.red_direct) {
+        k_reduce_quads<C><<<pl.quad_blocks, 4 * pl.quad_count, 0, stream>>>(inS, inW, qt, (int)nw, 1u << pl.quad_log2J,
+                                                                           span, terms);
         launches++;
         ZK_CUDA(cudaGetLastError());
     }
