@@ -424,6 +424,7 @@ static std::string autotune(Engine& e, int min_l2, int max_l2) {
     const size_t fb = P::N * 4;
     const uint64_t nmax = 1ull << max_l2;
     DevBuf pts, phi, sc, res;
+    for (DevBuf* b : {&pts, &phi, &sc, &res}) b->spare = &e.w_aff;
     pts.ensure(nmax * 2 * fb);
     phi.ensure(nmax * 2 * fb);
     sc.ensure(nmax * 32);
@@ -759,10 +760,12 @@ ZkMetalStatus zkmsm_table_create(ZkMetalMSMEngine engine, int curve, const void*
         Engine& e = ENG(engine);
         std::unique_ptr<Table> t(new Table{&e, curve, n, {}, {}});
         size_t bytes = (size_t)n * 2 * fp_bytes(curve);
+        t->points.spare = t->phi.spare = &e.w_aff;
         t->points.alloc_exact(bytes);
         with_curve(curve, [&](auto cv) {
             if (CurveTraits<decltype(cv)>::glv) t->phi.alloc_exact(bytes);
         });
+        t->points.spare = t->phi.spare = nullptr;  // the table may outlive the engine
         ZK_CUDA(cudaMemcpyAsync(t->points.p, points, bytes, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
                                 e.stream));
         with_curve(curve, [&](auto cv) {
@@ -791,6 +794,7 @@ ZkMetalStatus zkmsm_table_precompute(ZkMsmTable table, int spacing_bits) {
         Engine& e = *t.engine;
         const size_t ab = (size_t)2 * fp_bytes(t.curve);
         DevBuf nb;
+        nb.spare = &e.w_aff;
         nb.alloc_exact((size_t)copies * t.n * ab);
         ZK_CUDA(cudaMemcpyAsync(nb.p, t.points.p, (size_t)t.n * ab, cudaMemcpyDeviceToDevice, e.stream));
         with_curve(t.curve, [&](auto cv) { e.make_shifts<decltype(cv)>(nb.as<uint32_t>(), t.n, s, copies); });

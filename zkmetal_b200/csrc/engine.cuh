@@ -53,32 +53,56 @@ struct DevBuf {
     void* p = nullptr;
     size_t cap = 0;
     cudaStream_t* sp = nullptr;
+    // a buffer its owner can do without: given back when this one finds no memory
+    DevBuf* spare = nullptr;
+    // growth is geometric (at least 1.5x): a buffer that keeps growing is
+    // reallocated a logarithmic number of times
+    size_t grown(size_t bytes) const { return std::max(bytes + bytes / 8 + 256, cap + cap / 2); }
     bool ensure(size_t bytes) {  // true when it had to reallocate
         if (bytes <= cap) return false;
-        // growth is geometric (at least 1.5x): a buffer that keeps growing is
-        // reallocated a logarithmic number of times
-        size_t want = std::max(bytes + bytes / 8 + 256, cap + cap / 2);
+        const size_t want = grown(bytes);
         if (sp) {
             if (p) ZK_CUDA(cudaFreeAsync(p, *sp));
-            p = nullptr;
-            cap = 0;
-            ZK_CUDA(cudaMallocAsync(&p, want, *sp));
-        } else {
-            if (p) cudaFree(p);
-            p = nullptr;
-            cap = 0;
-            ZK_CUDA(cudaMalloc(&p, want));
+        } else if (p) {
+            cudaFree(p);
         }
-        cap = want;
+        p = nullptr;
+        cap = 0;
+        allocate(want);
         return true;
+    }
+    void allocate(size_t bytes) {
+        auto get = [&] { return sp ? cudaMallocAsync(&p, bytes, *sp) : cudaMalloc(&p, bytes); };
+        cudaError_t e = get();
+        if (e == cudaErrorMemoryAllocation && spare && spare->p) {
+            cudaGetLastError();
+            spare->give_back();
+            e = get();
+        }
+        if (e != cudaSuccess) {
+            p = nullptr;
+            throw CudaError{e, "growing a device buffer"};
+        }
+        cap = bytes;
+    }
+    // frees a stream-ordered buffer, its memory back to the device
+    void give_back() {
+        cudaFreeAsync(p, *sp);
+        p = nullptr;
+        cap = 0;
+        cudaStreamSynchronize(*sp);
+        int dev = 0;
+        cudaMemPool_t pool;
+        if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess)
+            cudaMemPoolTrimTo(pool, 0);
+        cudaGetLastError();
     }
     // exactly `bytes` (synchronous allocation, contents dropped): for
     // long-lived buffers such as resident tables, where growth slack would
     // waste gigabytes
     void alloc_exact(size_t bytes) {
         release();
-        ZK_CUDA(cudaMalloc(&p, bytes));
-        cap = bytes;
+        allocate(bytes);
     }
     template <class T>
     T* as() const { return static_cast<T*>(p); }
@@ -667,7 +691,10 @@ class Engine {
                           &w_pkeys[0], &w_pkeys[1], &w_pvals[0], &w_pvals[1], &w_redS[0], &w_redS[1],
                           &w_redW[0], &w_redW[1], &w_aff, &w_quad1, &w_quad2, &w_results, &w_comb, &w_profile, &transient.d_descs,
                           &transient.d_tasks};
-        for (DevBuf* b : bufs) b->sp = &stream;
+        for (DevBuf* b : bufs) {
+            b->sp = &stream;
+            if (b != &w_aff) b->spare = &w_aff;
+        }
         cudaMemPool_t pool;
         if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) {
             uint64_t keep = 4ull << 30, cur = 0;
@@ -1126,6 +1153,43 @@ class Engine {
         return transient;
     }
 
+    // The affine slab (up to 3.3 GB) only saves time: k_acc_l1 sums the same
+    // chunks without it.  So it is taken while it is at most an eighth of the
+    // memory the device has left, its pool's unused part included, and given
+    // back when another buffer of the engine finds none (DevBuf::spare).
+    static constexpr size_t AFF_MEMORY_SHARE = 8;
+    bool ensure_slab(size_t bytes) {  // true when the buffer moved or went
+        if (bytes <= w_aff.cap) return false;
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        size_t left = 0, total = 0;
+        uint64_t reserved = 0, used = 0;
+        cudaMemPool_t pool;
+        if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone ||
+            cudaMemGetInfo(&left, &total) != cudaSuccess ||
+            cudaDeviceGetDefaultMemPool(&pool, device) != cudaSuccess ||
+            cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+            cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        left += reserved - used + w_aff.cap;
+        if (w_aff.grown(bytes) > left / AFF_MEMORY_SHARE) return false;
+        const bool had = w_aff.p != nullptr;
+        try {
+            return w_aff.ensure(bytes);
+        } catch (const CudaError& e) {
+            if (e.code != cudaErrorMemoryAllocation) throw;
+            cudaGetLastError();
+            return had;
+        }
+    }
+    // The slab a plan's affine levels run in; null: there is none to be had
+    // and its chunks take k_acc_l1.
+    template <class P>
+    void* slab_of(const Plan& pl) const {
+        return pl.aff_levels && aff_layout<P>(pl).bytes <= w_aff.cap ? w_aff.p : nullptr;
+    }
+
     template <class C>
     void ensure_workspace(const Plan& pl) {
         using P = typename C::Fp;
@@ -1145,7 +1209,6 @@ class Engine {
         uint64_t m2 = 2, m3 = 2;
         if (pl.acc_Mbound.size() > 1) m2 = pl.acc_Mbound[1];
         for (size_t l = 2; l < pl.acc_Mbound.size(); l++) m3 = std::max<uint64_t>(m3, pl.acc_Mbound[l]);
-        if (pl.aff_levels) grew |= w_aff.ensure(aff_layout<P>(pl).bytes);
         grew |= w_pkeys[0].ensure(m2 * 4 + 16);
         grew |= w_pvals[0].ensure(m2 * xs + xs);
         grew |= w_pkeys[1].ensure(m3 * 4 + 16);
@@ -1164,6 +1227,7 @@ class Engine {
         grew |= w_results.ensure((pl.descs.size() + 1) * 3 * P::N * 4);
         // scan tile sums for the longest scanned array (no allocation inside enqueue)
         grew |= w_tiles.ensure(((std::max<uint64_t>(pl.nbuckets, hsz) + 2047) / 2048 + 2) * 4);
+        if (pl.aff_levels) grew |= ensure_slab(aff_layout<P>(pl).bytes);
         if (grew) {
             drop_graphs();  // captured graphs hold the old addresses
             workspace_growths++;
@@ -1279,6 +1343,7 @@ class Engine {
         put(d_phi);
         put(d_scalars);
         put(stream);
+        put(slab_of<P>(pl));  // another kernel sequence without one
         auto it = graphs.find(key);
         if (it == graphs.end()) {
             // the first call of a plan runs its launches directly: capturing

@@ -189,7 +189,7 @@ void Engine::enqueue(const Plan& pl, const uint32_t* d_bases, const uint32_t* d_
             k_acc_l1<C><<<(T - t0 + AT - 1) / AT, AT, 0, stream>>>(w_ents.as<uint2>(), d_len, K, t0, d_bases, d_phi,
                                                                   d_next, buckets, okeys, ovals);
         };
-        if (l == 0 && pl.aff_levels) {
+        if (l == 0 && slab_of<P>(pl)) {
           if constexpr (AFF_CURVE<C>) {
             const AffSlab sl = aff_slab<C>(pl);
             const uint32_t nb = sl.threads / AFF_THREADS;
@@ -217,7 +217,7 @@ void Engine::enqueue(const Plan& pl, const uint32_t* d_bases, const uint32_t* d_
                 level1((uint32_t)end);
             }
           }
-        } else if (l == 0 && !pl.acc_fold) {
+        } else if (l == 0 && !pl.acc_fold) {  // also affine plans that got no slab
             level1(0);
         } else if (l == 0) {
             k_acc_fold<C, true><<<T, FOLD_THREADS, 0, stream>>>(w_ents.as<uint2>(), d_bases, d_phi, nullptr, nullptr,
@@ -238,7 +238,7 @@ void Engine::enqueue(const Plan& pl, const uint32_t* d_bases, const uint32_t* d_
     prof_end(ev);
 }
 
-// The buffers of an affine slab inside w_aff (sized by aff_slab_bytes).
+// The buffers of an affine slab inside w_aff (aff_layout).
 template <class C>
 AffSlab Engine::aff_slab(const Plan& pl) const {
     const AffLayout a = aff_layout<typename C::Fp>(pl);
@@ -348,6 +348,7 @@ void Engine::make_shifts(uint32_t* d_table, uint64_t n, uint32_t s, uint32_t cop
     const uint64_t per_point = (uint64_t)(copies - 1) * sizeof(Xyzz<P>);
     const uint32_t m = (uint32_t)std::min<uint64_t>(n, std::max<uint64_t>(1024, (512ull << 20) / per_point));
     DevBuf scratch;
+    scratch.spare = &w_aff;
     scratch.ensure((size_t)m * per_point);
     Xyzz<P>* sc = scratch.as<Xyzz<P>>();
     for (uint64_t i0 = 0; i0 < n; i0 += m) {

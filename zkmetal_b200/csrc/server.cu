@@ -78,9 +78,24 @@ struct Server {
 
     static uint64_t estimate(int curve, uint32_t n) {
         // scalars + sorted entries (2 halves x up to 8 windows x 8 B) + buckets
-        // and partial sums; generous so admission errs on the safe side
+        // and partial sums; generous so admission errs on the safe side.  The
+        // slab of affine sums is not counted: where memory is short, an engine
+        // does without one (Engine::ensure_slab)
         const uint64_t per_point = 32 + 2 * 8 * 8 + (curve == ZKMSM_BN254 ? 64 : 96);
         return (uint64_t)n * per_point + (64ull << 20);
+    }
+
+    // Slab of affine sums of a worker's full BLS12-381 batches, by its largest
+    // entry count (shift-table windows of 4 bits: 64 entries per point).
+    uint64_t slab_bytes() const {
+        const uint64_t entries = max_batch_points * 64;
+        if (!has_table[1] || entries < AFF_MIN_ENTRIES) return 0;
+        Plan pl;
+        pl.aff_levels = 1;
+        pl.aff_threads = AFF_SLAB_DEFAULT;
+        const uint64_t K = std::min<uint64_t>(entries / AFF_SLAB_DEFAULT + 1, AFF_MAX_CHUNK);
+        pl.acc_K.push_back((uint32_t)(K + 3) / 4 * 4);
+        return aff_layout<Bls381::Fp>(pl).bytes;
     }
 
     void worker_main(int w) {
@@ -237,7 +252,8 @@ struct Server {
                     const DevBuf* ws[] = {&eng->w_ents, &eng->w_ents2,
                                           &eng->w_thist, &eng->w_buckets, &eng->w_pkeys[0],
                                           &eng->w_pkeys[1], &eng->w_pvals[0], &eng->w_pvals[1], &eng->w_redS[0],
-                                          &eng->w_redS[1], &eng->w_redW[0], &eng->w_redW[1], &eng->w_tiles};
+                                          &eng->w_redS[1], &eng->w_redW[0], &eng->w_redW[1], &eng->w_tiles,
+                                          &eng->w_aff, &eng->w_quad1, &eng->w_quad2};
                     uint64_t wsb = d_cap;
                     for (const DevBuf* b : ws) wsb += b->cap;
                     uint64_t pool_res = 0, pool_used = 0;
@@ -467,18 +483,13 @@ ZkMetalStatus zkmsm_server_create(ZkMsmTable bn254_table, ZkMsmTable bls12_381_t
     // without mapping.  A worker's workspace for a full batch of small and
     // medium MSMs over window-shift tables (one sorted entry per window per
     // point, two entry arrays, scalars) reaches about 480 B per batch point;
-    // BLS12-381 batches add a slab of affine sums, 86 B for each of at most
-    // 13 entries per point and one wave of the longest chunks.
+    // BLS12-381 batches add a slab of affine sums.
     {
         size_t fr = 0, tot = 0;
         cudaMemPool_t pool;
         if (cudaMemGetInfo(&fr, &tot) == cudaSuccess && cudaDeviceGetDefaultMemPool(&pool, s->device) == cudaSuccess) {
-            const uint64_t slab =
-                    bls12_381_table
-                            ? std::min<uint64_t>(s->max_batch_points * 13, (uint64_t)AFF_SLAB_DEFAULT * AFF_MAX_CHUNK) * 86
-                            : 0;
-            const uint64_t want =
-                    std::min<uint64_t>((uint64_t)workers * (s->max_batch_points * 512 + slab) + (1ull << 30), fr / 4);
+            const uint64_t want = std::min<uint64_t>(
+                    (uint64_t)workers * (s->max_batch_points * 512 + s->slab_bytes()) + (1ull << 30), fr / 4);
             uint64_t thr = 0;
             cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
             if (thr < want) {
