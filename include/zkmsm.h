@@ -355,6 +355,12 @@ ZkMetalStatus zkmsm_engine_phase_times(ZkMetalMSMEngine engine, double* ms5, uin
  * computation: no device is touched. */
 ZkMetalStatus zkmsm_plan_describe(int curve, const uint32_t* counts, uint32_t n_msms, int scalar_fmt,
                                   int window_bits, int chunk, int glv, int scalar_bits, char* buf, uint64_t buflen);
+/* The same for one MSM of n points whose scalars were sampled (window_bits as
+ * chosen from the sample, expected_entries sorted entries; 0: not sampled),
+ * with an autotuned chunk length of chunk_pct percent of the rule's (0: the
+ * rule's). */
+ZkMetalStatus zkmsm_plan_describe_sampled(int curve, uint32_t n, int scalar_fmt, int window_bits,
+                                          uint64_t expected_entries, int chunk_pct, char* buf, uint64_t buflen);
 /* The same for MSMs over prefixes of a table of table_points points with
  * window shifts of spacing shift_bits (zkmsm_table_precompute). */
 ZkMetalStatus zkmsm_plan_describe_shift(int curve, const uint32_t* counts, uint32_t n_msms, int scalar_fmt,

@@ -108,3 +108,17 @@ def test_affine_slabs_past_the_expected_entries(engines):
     v[::512] = 0
     a = run(e, pts, sc, n, zl.SCALAR_MONT, 0)
     assert a == run(e, pts, sc, n, zl.SCALAR_MONT, 64)
+
+
+@pytest.mark.parametrize("pct", [50, 200])
+def test_affine_tuned_chunks(engines, tmp_path, pct):
+    """Chunk lengths from a saved schedule: more slabs, or longer chunks."""
+    n = (1 << 19) + 5
+    path = tmp_path / "tuning"
+    path.write_text("zkmsm-tuning 2\n" + "s %d 19 %d 0 0\n" % (zl.BLS12_381 * 2 + 1, pct))
+    pts, sc = gen_inputs(engines["bls12_381"], "bls12_381", 93, n, "uniform", zl.SCALAR_MONT)
+    e = BLS12381MSM()
+    check(zl.lib().zkmsm_tuning_load(e.handle, str(path).encode()))
+    got = run(e, pts, sc, n, zl.SCALAR_MONT, 0)
+    e.close()
+    assert got == run(engines["bls12_381"], pts, sc, n, zl.SCALAR_MONT, 64)

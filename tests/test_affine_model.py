@@ -156,3 +156,38 @@ def test_plan_rule(curve, n):
         # halved while more than one and a half long
         assert K >> levels >= 4 and 2 * run >= 3 << (levels - 1)
     assert describe(curve, n, chunk=64)["affine"] == [0, 0, 0]
+
+
+def describe_sampled(curve, n, window=0, entries=0, pct=0):
+    buf = ctypes.create_string_buffer(1 << 22)
+    assert zl.lib().zkmsm_plan_describe_sampled(curve, n, 1, window, entries, pct, buf, len(buf)) == 0
+    return json.loads(buf.value.decode())
+
+
+@pytest.mark.parametrize("curve", [zl.BLS12_381, zl.BLS12_377, zl.BN254_G2])
+@pytest.mark.parametrize("n", [1 << 18, 1 << 20, 3000001, 1 << 22])
+@pytest.mark.parametrize("pct", [10, 50, 99, 100, 200, 1000])
+def test_plan_rule_with_tuned_chunks(curve, n, pct):
+    """An autotuned chunk length changes the affine chunks, and the slabs
+    still hold all of them."""
+    rule, pl = describe_sampled(curve, n), describe_sampled(curve, n, pct=pct)
+    levels, threads, slabs = pl["affine"]
+    K, T, M = pl["acc"][0]
+    assert levels and rule == describe(curve, n)
+    assert 16 <= K <= 512 and K % 4 == 0
+    want = min(512, max(16, rule["acc"][0][0] * pct // 100))
+    assert abs(K - want) <= 4 + 3 * pct // 100
+    assert slabs * threads >= T > (slabs - 1) * threads, "chunks outside the slabs are none of the affine levels"
+
+
+@pytest.mark.parametrize("n,entries", [(1 << 21, 8390000), (1 << 22, 1 << 23), (1 << 20, 5000000)])
+def test_plan_rule_with_few_expected_entries(n, entries):
+    """A sample that expects fewer entries than the bound: slabs for those,
+    and chunks past them for k_acc_l1."""
+    pl = describe_sampled(zl.BLS12_381, n, 15, entries)
+    levels, threads, slabs = pl["affine"]
+    K, T, M = pl["acc"][0]
+    assert levels and M > entries
+    assert slabs * threads * K >= entries > (slabs - 1) * threads * K
+    assert T == -(-M // K) > slabs * threads
+    assert describe_sampled(zl.BLS12_381, n, 15, (1 << 22) - 1)["affine"] == [0, 0, 0]

@@ -1006,7 +1006,8 @@ ZkMetalStatus zkmsm_engine_phase_times(ZkMetalMSMEngine engine, double* ms5, uin
 }
 
 static ZkMetalStatus plan_json(int curve, const uint32_t* counts, uint32_t n_msms, int fmt, int window_bits,
-                               int chunk, int glv, int scalar_bits, ShiftSpec sh, char* buf, uint64_t buflen) {
+                               int chunk, int glv, int scalar_bits, ShiftSpec sh, uint64_t entries_hint, int chunk_pct,
+                               char* buf, uint64_t buflen) {
     if (!counts || !buf || n_msms == 0 || !window_setting_ok(window_bits)) return ZKMETAL_ERR_INVALID_INPUT;
     return guarded([&] {
         Tuning t;
@@ -1015,8 +1016,12 @@ static ZkMetalStatus plan_json(int curve, const uint32_t* counts, uint32_t n_msm
         t.glv = glv;
         std::vector<uint32_t> cnt(counts, counts + n_msms), boff(n_msms, 0);
         Plan pl;
+        if (chunk_pct > 0)
+            for (int g = 0; g < 2; g++)
+                for (auto n : cnt)
+                    if (n) t.sched_table[{curve * 2 + g, nearest_log2(n)}].chunk_pct = chunk_pct;
         with_curve(curve, [&](auto cv) {
-            Engine::plan_shape<decltype(cv)>(pl, t, cnt, boff, fmt, scalar_bits, 0, sh);
+            Engine::plan_shape<decltype(cv)>(pl, t, cnt, boff, fmt, scalar_bits, 0, sh, entries_hint);
         });
         std::string s = "{\"descs\":[";
         for (size_t i = 0; i < pl.descs.size(); i++) {
@@ -1068,7 +1073,13 @@ static ZkMetalStatus plan_json(int curve, const uint32_t* counts, uint32_t n_msm
 
 ZkMetalStatus zkmsm_plan_describe(int curve, const uint32_t* counts, uint32_t n_msms, int fmt, int window_bits,
                                   int chunk, int glv, int scalar_bits, char* buf, uint64_t buflen) {
-    return plan_json(curve, counts, n_msms, fmt, window_bits, chunk, glv, scalar_bits, ShiftSpec{}, buf, buflen);
+    return plan_json(curve, counts, n_msms, fmt, window_bits, chunk, glv, scalar_bits, ShiftSpec{}, 0, 0, buf, buflen);
+}
+
+ZkMetalStatus zkmsm_plan_describe_sampled(int curve, uint32_t n, int fmt, int window_bits, uint64_t expected_entries,
+                                          int chunk_pct, char* buf, uint64_t buflen) {
+    if (!curve_ok(curve) || !n || chunk_pct < 0) return ZKMETAL_ERR_INVALID_INPUT;
+    return plan_json(curve, &n, 1, fmt, window_bits, 0, -1, 0, ShiftSpec{}, expected_entries, chunk_pct, buf, buflen);
 }
 
 ZkMetalStatus zkmsm_plan_describe_shift(int curve, const uint32_t* counts, uint32_t n_msms, int fmt,
@@ -1076,7 +1087,7 @@ ZkMetalStatus zkmsm_plan_describe_shift(int curve, const uint32_t* counts, uint3
                                         uint64_t buflen) {
     if (shift_bits < 2 || shift_bits > 24) return ZKMETAL_ERR_INVALID_INPUT;
     return plan_json(curve, counts, n_msms, fmt, window_bits, 0, -1, 0,
-                     ShiftSpec{(uint32_t)shift_bits, table_points}, buf, buflen);
+                     ShiftSpec{(uint32_t)shift_bits, table_points}, 0, 0, buf, buflen);
 }
 
 uint64_t zkmsm_engine_launch_count(ZkMetalMSMEngine engine) { return engine ? ENG(engine).launches : 0; }

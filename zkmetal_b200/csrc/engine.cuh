@@ -969,10 +969,10 @@ class Engine {
                 W = std::max(AFF_SLAB_UNIT, (W ? W : AFF_SLAB_DEFAULT) / AFF_SLAB_UNIT * AFF_SLAB_UNIT);
                 const uint64_t slabs = (Me + (uint64_t)W * AFF_MAX_CHUNK - 1) / ((uint64_t)W * AFF_MAX_CHUNK);
                 K1 = (uint32_t)((Me + slabs * W - 1) / (slabs * W));
-                if (sc.chunk_pct > 0) K1 = std::min<uint32_t>(2 * AFF_MAX_CHUNK, K1 * sc.chunk_pct / 100);
-                K1 = std::max<uint32_t>((K1 + 3) / 4 * 4, 16);
+                if (sc.chunk_pct > 0) K1 = K1 * sc.chunk_pct / 100;
+                K1 = std::min<uint32_t>(std::max<uint32_t>((K1 + 3) / 4 * 4, 16), AFF_MAX_CHUNK);
                 pl.aff_threads = W;
-                pl.aff_slabs = (uint32_t)slabs;
+                pl.aff_slabs = (uint32_t)((Me + (uint64_t)K1 * W - 1) / ((uint64_t)K1 * W));
                 while (pl.aff_levels < 8 && (K1 >> (pl.aff_levels + 1)) >= 4 &&
                        2 * run >= (3ull << pl.aff_levels))  // 1.5 per run left to halve
                     pl.aff_levels++;
