@@ -123,3 +123,12 @@ def test_quad_reduction_many_windows(counts):
         warps = sum(-(-min(n, 64 << Q["log2J"]) // (8 << Q["log2J"])) for n in nodes)
         assert 8 * warps <= 2 * (sum(nodes) >> Q["log2J"]) + 8 * len(nodes)
     check(pl, len(counts))
+
+
+@pytest.mark.parametrize("counts", [[0], [0] * 3, [0, 1], [1]])
+def test_plan_of_few_entries(counts):
+    """A batch of empty MSMs has no entries: its one segmented-sum level is
+    the shortest there is."""
+    pl = plan(zl.BN254, counts)
+    K, T, M = pl["acc"][0]
+    assert M == pl["entry_bound"] and K == QUADS * 4 and T == 1 and len(pl["acc"]) == 1

@@ -985,9 +985,10 @@ class Engine {
         // 4119 and 4057 us for the whole call; BLS12-377 10^5 1781 and 1751)
         const uint64_t fb = tuning.fold_blocks[CurveTraits<C>::id] ? tuning.fold_blocks[CurveTraits<C>::id] : 296;
         auto fold_chunk = [fb](uint64_t m) {
+            m = std::max<uint64_t>(m, 1);  // a batch of empty MSMs has no entries
             const uint64_t wave = FOLD_QUADS * fb;  // quads resident
             const uint64_t waves = (m + wave * FOLD_MAX_J - 1) / (wave * FOLD_MAX_J);
-            const uint64_t J = (m + wave * waves - 1) / (wave * std::max<uint64_t>(waves, 1));
+            const uint64_t J = (m + wave * waves - 1) / (wave * waves);
             return FOLD_QUADS * (uint32_t)std::max<uint64_t>(4, (J + 1) / 2 * 2);
         };
         pl.acc_fold = tuning.chunk <= 0 && M <= ACC_FOLD_MAX_ENTRIES;
