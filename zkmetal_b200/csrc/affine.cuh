@@ -64,6 +64,8 @@ struct AffSlab {
     uint32_t* cnt;     // [thread]: elements
     uint32_t* npair;   // [thread]: pairs of this level
     uint32_t K, pcap, threads;  // K a multiple of 4, pcap = K / 2
+    uint32_t slabs;    // that the expected entries fill, at chunks of K
+    uint32_t chunks;   // of K for all the entries there may be
 };
 
 // A point in memory: words `step` apart, y negated or not.
@@ -135,6 +137,15 @@ __device__ __noinline__ Fe<P> aff_look_d(Fe<P> d, const AffPoint a, const AffPoi
     if (b.neg) fe_neg(v.y, v.y);
     aff_special_d(d, u, v);
     return d;
+}
+
+// Chunk length for M entries: as acc_chunk, whole slabs of at most K; K when the
+// slabs hold too few (the chunks after them are k_acc_l1's).
+ZK_DEV uint32_t aff_len(const AffSlab& s, uint32_t M) {
+    const uint64_t per = (uint64_t)s.K * s.threads;
+    if (M == 0 || M > per * s.slabs) return s.K;
+    const uint64_t parts = min((M + per - 1) / per * s.threads, (uint64_t)s.chunks);
+    return min(s.K, max(16u, (uint32_t)((M + 4 * parts - 1) / (4 * parts)) * 4));
 }
 
 // Entries of chunk g: [g*K, ..) of M.
@@ -238,8 +249,9 @@ __global__ void __launch_bounds__(AFF_THREADS, AffLaunch<C>::BLOCKS) k_aff_pair(
     uint4* my = ring + threadIdx.x * AffRing<P>::SLOT;
     const size_t warp = t >> 5, lane = t & 31;
     const uint64_t g = g0 + t;
-    const uint32_t n = FIRST ? aff_chunk(g, s.K, *d_len) : s.cnt[t];
-    const uint2* en = ents + g * s.K;
+    const uint32_t M = FIRST ? *d_len : 0, K = FIRST ? aff_len(s, M) : 0;
+    const uint32_t n = FIRST ? aff_chunk(g, K, M) : s.cnt[t];
+    const uint2* en = ents + g * K;
     const uint4* pts = s.pts + warp * s.pcap * (2 * V) * 32 + lane;
     uint4* pre = s.pre + warp * s.pcap * V * 32 + lane;
     uint2* info = s.info + warp * s.pcap * 32 + lane;
@@ -517,9 +529,9 @@ __global__ void __launch_bounds__(AFF_THREADS) k_aff_finish(
     if (t >= s.threads) return;
     const size_t warp = t >> 5, lane = t & 31;
     const uint64_t g = g0 + t;
-    const uint32_t M = *d_len;
-    if (g == 0) *d_next = (uint32_t)(2 * (((uint64_t)M + s.K - 1) / s.K));
-    if (!aff_chunk(g, s.K, M)) return;
+    const uint32_t M = *d_len, K = aff_len(s, M);
+    if (g == 0) *d_next = (uint32_t)(2 * (((uint64_t)M + K - 1) / K));
+    if (!aff_chunk(g, K, M)) return;
     const uint32_t n = s.cnt[t];
     const uint4* pts = s.pts + warp * s.pcap * (2 * P::N / 4) * 32 + lane;
     const uint2* runs = s.runs + warp * s.K * 32 + lane;

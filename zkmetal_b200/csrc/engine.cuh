@@ -296,6 +296,8 @@ struct Plan {
     // threads (chunks) of a slab, and the slabs the expected entries fill
     // (chunks past them, if there are more entries, take k_acc_l1)
     uint32_t aff_levels = 0, aff_threads = 0, aff_slabs = 0;
+    // threads of k_acc_l1 resident at once (0: unknown, or the chunk length is forced)
+    uint32_t acc_wave = 0;
     std::vector<uint32_t> acc_K, acc_T;
     std::vector<uint64_t> acc_Mbound;
     // bucket-reduction tree (levels of arity red_L to one node per window); the
@@ -334,6 +336,7 @@ struct Plan {
         red_L = 8;
         red_log2L = 3;
         acc_threads = 0;
+        acc_wave = 0;
         acc_fold = false;
         aff_levels = aff_threads = aff_slabs = 0;
         acc_K.clear();
@@ -928,6 +931,7 @@ class Engine {
         uint64_t M = pl.entry_bound;
         uint32_t K1 = tuning.chunk > 0 ? (uint32_t)tuning.chunk : 0;
         if (!K1) {
+            pl.acc_wave = tuning.acc_wave[CurveTraits<C>::id];
             // long enough to hold about two average buckets and at least 192
             // entries (so few buckets are cut and the partial-sum levels stay
             // small: at 2^24 with ~24 entries per bucket, chunks of 192 beat

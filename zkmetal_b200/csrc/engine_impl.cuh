@@ -182,12 +182,12 @@ void Engine::enqueue(const Plan& pl, const uint32_t* d_bases, const uint32_t* d_
         uint32_t* okeys = w_pkeys[cur].as<uint32_t>();
         Xyzz<P>* ovals = w_pvals[cur].as<Xyzz<P>>();
         // k_acc_l1 over chunks [t0, T)
-        auto level1 = [&](uint32_t t0) {
+        auto level1 = [&](uint32_t t0, uint32_t wave) {
             const uint32_t AT = pl.acc_threads && pl.acc_threads <= (uint32_t)AccLaunch<C>::THREADS
                                         ? pl.acc_threads
                                         : (uint32_t)AccLaunch<C>::THREADS;
-            k_acc_l1<C><<<(T - t0 + AT - 1) / AT, AT, 0, stream>>>(w_ents.as<uint2>(), d_len, K, t0, d_bases, d_phi,
-                                                                  d_next, buckets, okeys, ovals);
+            k_acc_l1<C><<<(T - t0 + AT - 1) / AT, AT, 0, stream>>>(w_ents.as<uint2>(), d_len, K, T, wave, t0, d_bases,
+                                                                  d_phi, d_next, buckets, okeys, ovals);
         };
         if (l == 0 && slab_of<P>(pl)) {
           if constexpr (AFF_CURVE<C>) {
@@ -214,11 +214,11 @@ void Engine::enqueue(const Plan& pl, const uint32_t* d_bases, const uint32_t* d_
             }
             if (end < T) {
                 launches++;
-                level1((uint32_t)end);
+                level1((uint32_t)end, 0);
             }
           }
         } else if (l == 0 && !pl.acc_fold) {  // also affine plans that got no slab
-            level1(0);
+            level1(0, pl.acc_wave);
         } else if (l == 0) {
             k_acc_fold<C, true><<<T, FOLD_THREADS, 0, stream>>>(w_ents.as<uint2>(), d_bases, d_phi, nullptr, nullptr,
                                                                 d_len, K / FOLD_QUADS, last, d_next, buckets, okeys,
@@ -255,6 +255,8 @@ AffSlab Engine::aff_slab(const Plan& pl) const {
     s.K = pl.acc_K[0];
     s.pcap = a.pcap;
     s.threads = pl.aff_threads;
+    s.slabs = pl.aff_slabs;
+    s.chunks = pl.acc_T[0];
     return s;
 }
 

@@ -910,9 +910,24 @@ template <>
 struct AccLaunch<Bls377> {  // the same 12-limb arithmetic as BLS12-381
     static constexpr int THREADS = 256, MIN_BLOCKS = 2;
 };
+
+// Chunk length for M entries where the plan has T chunks of K for the entries
+// there may be.  Zero digits leave fewer (a third, witness-like scalars), and
+// chunks of K would then fill part of a wave of resident threads (wave; 0: K
+// whatever M is).  So the entries go to whole waves, in chunks of at most K and
+// at most T of them.  BN254, witness-like scalars, K throughout and now: 600001
+// points 1630 and 1136 us, 1024 MSMs of 1024 points 7371 and 5633 us.
+ZK_DEV uint32_t acc_chunk(uint32_t M, uint32_t K, uint32_t T, uint32_t wave) {
+    const uint64_t per = (uint64_t)K * wave;
+    if (per == 0 || M == 0) return K;
+    const uint64_t parts = min((M + per - 1) / per * wave, (uint64_t)T);
+    return max(8u, (uint32_t)((M + parts - 1) / parts));
+}
+
 template <class C>
 __global__ void __launch_bounds__(AccLaunch<C>::THREADS, AccLaunch<C>::MIN_BLOCKS) k_acc_l1(const uint2* __restrict__ ents,
-                                                const uint32_t* __restrict__ d_len, uint32_t K, uint32_t t0,
+                                                const uint32_t* __restrict__ d_len, uint32_t K, uint32_t T,
+                                                uint32_t wave, uint32_t t0,
                                                 const uint32_t* __restrict__ bases,
                                                 const uint32_t* __restrict__ phi,
                                                 uint32_t* __restrict__ d_next,
@@ -922,6 +937,7 @@ __global__ void __launch_bounds__(AccLaunch<C>::THREADS, AccLaunch<C>::MIN_BLOCK
     using P = typename C::Fp;
     uint32_t t = t0 + blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t M = *d_len;
+    K = acc_chunk(M, K, T, wave);
     if (t == 0) *d_next = (uint32_t)(2 * (((uint64_t)M + K - 1) / K));
     uint64_t start64 = (uint64_t)t * K;
     if (start64 >= M) return;
