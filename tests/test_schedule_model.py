@@ -2,13 +2,14 @@
 
 The plan (window widths, bucket layout, segmented-sum chunking, reduction
 tree) comes from the C++ planner through zkmsm_plan_describe.  The kernels'
-index logic -- histogram, exclusive scan, counting-sort scatter (in a
-shuffled order, as atomics allow), chunked segmented sums with their partial
-slots, the multi-level partial passes, the weighted reduction tree and the
-Horner combine -- is replayed here with integers mod r standing in for group
-elements (P_i -> p_i, phi(P) -> lambda*p).  Every index is checked against the
-sizes the engine allocates from the same plan, every bucket must be written
-at most once, and the result must equal sum s_i p_i mod r.  No GPU needed.
+index logic -- the entries in bucket order (shuffled within a bucket, as
+atomics allow), k_acc_l1's chunks with their two fixed slots, k_acc_fold's
+leaves, quads and merges on every level after it, the bucket reduction by
+levels and quads, and the windows' shifted sum -- is replayed here with
+integers mod r standing in for group elements (P_i -> p_i, phi(P) ->
+lambda*p).  Every index is checked against the sizes the engine allocates from
+the same plan, every bucket with entries must be written exactly once and no
+other, and the result must equal sum s_i p_i mod r.  No GPU needed.
 """
 import ctypes
 import json
@@ -65,12 +66,75 @@ def digits(k, c, nwin, nlo=None):
             carry = 0
 
 
-def excl_scan(a):
-    out, run = [], 0
-    for v in a:
-        out.append(run)
-        run += v
-    return out, run
+EMPTY = None  # ACC_EMPTY
+FOLD_QUADS = 64
+
+
+class Node:
+    """FoldNode: the first and last run of a range (one run when `whole`)."""
+
+    def __init__(self, kl=EMPTY, l=0):
+        self.kl, self.l, self.kr, self.r, self.whole = kl, l, EMPTY, 0, True
+
+
+def fold_merge(a, b, write):
+    """a ++ b, runs that end inside written to their buckets."""
+    if b.kl is EMPTY:
+        return a
+    if a.kl is EMPTY:
+        return b
+    ka, s = (a.kl, a.l) if a.whole else (a.kr, a.r)
+    same = ka == b.kl
+    if same:
+        s = s + b.l
+    o = Node(a.kl, a.l)
+    o.kr, o.r, o.whole = a.kr, a.r, a.whole
+    if not a.whole and not (same and b.whole):
+        write(ka, s)
+    if not same and not b.whole:
+        write(b.kl, b.l)
+    if same and a.whole:
+        o.l = s
+    if same and b.whole:
+        if not a.whole:
+            o.r = s
+    else:
+        o.kr, o.r = (b.kl, b.l) if b.whole else (b.kr, b.r)
+        o.whole = False
+    return o
+
+
+def fold_block(leaves, J, write):
+    """One block of k_acc_fold: `leaves` of its FOLD_QUADS * J places."""
+    nodes = []
+    for i in range(FOLD_QUADS):
+        a = Node()
+        for key, val in leaves[i * J:(i + 1) * J]:
+            a = fold_merge(a, Node(key, val), write)
+        nodes.append(a)
+    st = 1
+    while st < FOLD_QUADS:  # three steps inside the warps, three over them
+        for i in range(0, FOLD_QUADS, 2 * st):
+            nodes[i] = fold_merge(nodes[i], nodes[i + st], write)
+        st *= 2
+    return nodes[0]
+
+
+def acc_l1(entries, K, write):
+    """k_acc_l1: slots 2t and 2t + 1 take chunk t's first and last run."""
+    slots = []
+    for start in range(0, len(entries), K):
+        chunk = entries[start:start + K]
+        runs = []
+        for k, v in chunk:
+            if runs and runs[-1][0] == k:
+                runs[-1] = (k, runs[-1][1] + v)
+            else:
+                runs.append((k, v))
+        for k, v in runs[1:-1]:
+            write(k, v)
+        slots += [runs[0], runs[-1] if len(runs) > 1 else (EMPTY, 0)]
+    return slots
 
 
 def plan_shift(curve, counts, shift_bits, table_points, window=0):
@@ -82,7 +146,7 @@ def plan_shift(curve, counts, shift_bits, table_points, window=0):
     return json.loads(buf.value.decode())
 
 
-def run_model(C, pl, bases, scalars, seed=0):
+def run_model(C, pl, bases, scalars, seed=0, chunk=0):
     """`bases`: the base table as the entries index it (for a shift-table
     plan, copy k of the table at k * table_points + i)."""
     r = C.r
@@ -90,7 +154,7 @@ def run_model(C, pl, bases, scalars, seed=0):
     rng = random.Random(seed)
     descs = pl["descs"]
     G = pl["nbuckets"]
-    # 1-3: histogram, scan, scatter
+    # 1-3: digits, sort
     entries = []
     for d in descs:
         soff, n, boff, c, nwin, glv, bucket_off, fmt, win_off, wstep, nred, nlo = d
@@ -127,87 +191,43 @@ def run_model(C, pl, bases, scalars, seed=0):
         written[k] = True
         buckets[k] = x % r
 
-    cur_keys, cur_vals = keys, None
-    M = len(keys)
+    # 4: segmented sums
+    assert pl["affine"][0] == 0
+    lst = [(k, point(v)) for k, v in zip(keys, vals)]
+    fold = pl["entry_bound"] <= 1 << 16 and not chunk
     for lvl, (K, T, Mbound) in enumerate(pl["acc"]):
-        assert M <= Mbound
-        cnt = []
-        for t in range(T):
-            start = t * K
-            if start >= M:
-                cnt.append(0)
-                continue
-            end = min(start + K, M)
-            k0, k1 = cur_keys[start], cur_keys[end - 1]
-            cb = int(start > 0 and cur_keys[start - 1] == k0)
-            ca = int(end < M and cur_keys[end] == k1)
-            cnt.append((cb | ca) if k0 == k1 else cb + ca)
-        pos, total = excl_scan(cnt)
-        if lvl + 1 < len(pl["acc"]):
-            assert total <= pl["acc"][lvl + 1][2], "partial slots exceed the next level's bound"
+        M, last = len(lst), lvl + 1 == len(pl["acc"])
+        assert M <= Mbound and T == max(1, -(-Mbound // K))
+        if lvl == 0 and not fold:
+            assert not last
+            lst = acc_l1(lst, K, write_bucket)
         else:
-            assert total == 0, "last level must complete every bucket"
-        pkeys = [None] * total
-        pvals = [None] * total
-        for t in range(T):
-            start = t * K
-            if start >= M:
-                continue
-            end = min(start + K, M)
-            cur = cur_keys[start]
-            cont_before = start > 0 and cur_keys[start - 1] == cur
-            first_run = True
-            slot = pos[t]
-            acc = 0
-            for i in range(start, end):
-                k = cur_keys[i]
-                if k != cur:
-                    if first_run and cont_before:
-                        pkeys[slot], pvals[slot] = cur, acc
-                        slot += 1
-                    else:
-                        write_bucket(cur, acc)
-                    acc, cur, first_run = 0, k, False
-                acc += point(vals[i]) if lvl == 0 else cur_vals[i]
-            cont_after = end < M and cur_keys[end] == cur
-            if (first_run and cont_before) or cont_after:
-                assert slot < total
-                pkeys[slot], pvals[slot] = cur, acc
-                slot += 1
-            else:
-                write_bucket(cur, acc)
-            assert slot == pos[t] + cnt[t], "slot count disagrees with the chunk count pass"
-        cur_keys, cur_vals, M = pkeys, pvals, total
-    assert M == 0
-    # bucket reduction tree
-    L, log2L = pl["red_L"], pl["red_log2L"]
-    inS, inW = buckets, None
-    for lvl, tasks in enumerate(pl["red"]):
-        nout = sum(t[3] for t in tasks)
-        outS, outW = [None] * nout, [None] * nout
-        for (in_off, n_in, out_off, n_out) in tasks:
-            for local in range(n_out):
-                g = out_off + local
-                c0 = in_off + local * L
-                cnt = min(L, n_in - local * L)
-                run = x = 0
-                for s in range(cnt - 1, 0, -1):
-                    run += inS[c0 + s]
-                    x += run
-                run += inS[c0]
-                outS[g] = run % r
-                x = x * (1 << (lvl * log2L))
-                if inW is not None:
-                    x += sum(inW[c0 + s] for s in range(cnt))
-                outW[g] = x % r
-        inS, inW = outS, outW
+            assert K % FOLD_QUADS == 0
+            out = []
+            for blk in range(0, M, K):
+                a = fold_block(lst[blk:blk + K], K // FOLD_QUADS, write_bucket)
+                if last:
+                    assert a.kl is not EMPTY
+                    write_bucket(a.kl, a.l)
+                    if not a.whole:
+                        write_bucket(a.kr, a.r)
+                else:
+                    out += [(a.kl, a.l), (EMPTY, 0) if a.whole else (a.kr, a.r)]
+            lst = out
+        assert len(lst) == (0 if last else 2 * -(-M // K))
+        if last:
+            assert T == 1
+        else:
+            assert len(lst) <= pl["acc"][lvl + 1][2]
+    assert {k for k in range(G) if written[k]} == set(keys)
+    # 5: bucket reduction and the windows' sum
+    from tests.test_quad_reduce_model import reduce_model
+    wins = reduce_model(pl, buckets)
     results = []
     for d in descs:
         soff, n, boff, c, nwin, glv, bucket_off, fmt, win_off, wstep, nred, nlo = d
         assert nred == (1 if wstep else nwin)
-        acc = 0
-        for w in range(nred - 1, -1, -1):
-            acc = acc * (1 << win_width(c, nlo, w)) + inS[win_off + w] + inW[win_off + w]
+        acc = sum(wins[win_off + w] << (0 if wstep else win_bit(c, nlo, w)) for w in range(nred))
         results.append(acc % r if n else 0)
     return results
 
@@ -217,6 +237,8 @@ CASES = [
     ("bn254", [700], "uniform", 0, 0, -1, 0),
     ("bn254", [700], "witness", 0, 8, -1, 0),
     ("bn254", [2000], "witness", 6, 8, -1, 0),        # hot buckets -> several partial levels
+    ("bn254", [2000], "witness", 7, 0, -1, 0),        # entry sets above the fold threshold: k_acc_l1 first
+    ("bn254", [900, 40] * 3, "uniform", 0, 0, -1, 0),
     ("bn254", [300, 0, 17, 1, 900], "uniform", 0, 0, -1, 0),
     ("bn254", [500], "uniform", 11, 33, 0, 0),          # no GLV: 255-bit scalars
     ("bn254", [400], "uniform", 0, 0, -1, 16),          # small-scalar plan
@@ -245,7 +267,7 @@ def test_schedule_model(curve, counts, dist, window, chunk, glv, bits):
         for _ in range(total):
             u = rng.randrange(100)
             scalars.append(0 if u < 40 else 1 if u < 60 else rng.getrandbits(32) if u < 85 else rng.randrange(C.r))
-    got = run_model(C, pl, bases, scalars, seed=len(counts))
+    got = run_model(C, pl, bases, scalars, seed=len(counts), chunk=chunk)
     off = 0
     for m, n in enumerate(counts):
         # the plan puts every MSM on a prefix of one base table (base_off = 0)
@@ -267,7 +289,7 @@ LAYOUT_CASES = [
 @pytest.mark.parametrize("curve,counts,dist,c,nlo", LAYOUT_CASES)
 def test_schedule_model_two_width(curve, counts, dist, c, nlo):
     """Forced two-width layouts (window setting c | nlo << 16): digits,
-    bucket offsets, reduction tasks and the Horner combine per window width."""
+    bucket offsets, reduction tasks and the windows' shifts per window width."""
     C = R.CURVES[curve]
     cid = zl.BN254 if curve == "bn254" else zl.BLS12_381
     pl = plan(cid, counts, 0, c | (nlo << 16), 0, -1, 0)
