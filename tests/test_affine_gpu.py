@@ -98,16 +98,34 @@ def test_affine_levels(engines, oracles, curve, n, kind):
 
 
 def test_affine_slabs_past_the_expected_entries(engines):
-    """A sampled layout expects few entries (mostly zero scalars in the
-    sample's places); the chunks past its slabs take k_acc_l1."""
-    e = engines["bls12_381"]
+    """A sampled plan expects a third of the entries there are: two in three
+    of the scalars the sample reads (every 512th of 2^21) are zero, no other.
+    The chunks past its slabs take k_acc_l1."""
+    e, L = engines["bls12_381"], zl.lib()
     n = 1 << 21
     pts, sc = gen_inputs(e, "bls12_381", 92, n, "uniform", zl.SCALAR_MONT)
-    v = sc.view(n, 32)
-    v[::2] = 0  # the sample reads every 512th scalar: it sees zeros only in part
-    v[::512] = 0
-    a = run(e, pts, sc, n, zl.SCALAR_MONT, 0)
-    assert a == run(e, pts, sc, n, zl.SCALAR_MONT, 64)
+    v = sc.view(n // 512, 512, 32)
+    zero = torch.arange(n // 512, device="cuda") % 3 != 0
+    v[zero, 0] = 0
+    few = sc.clone()  # the same sample, and as few entries as it promises
+    few.view(n // 512, 512, 32)[zero] = 0
+
+    def counted(scalars, chunk):
+        k = L.zkmsm_engine_launch_count(e.handle)
+        out = run(e, pts, scalars, n, zl.SCALAR_MONT, chunk)
+        return out, L.zkmsm_engine_launch_count(e.handle) - k, L.zkmsm_engine_last_entries(e.handle)
+
+    got, launches, entries = counted(sc, 0)
+    _, same, expected = counted(few, 0)
+    # one plan for both, in affine levels (two and more launch six kernels);
+    # its slabs hold the expected entries and at most a tenth more
+    assert launches == same and launches >= counted(sc, 64)[1] + 6
+    assert expected >= 1 << 22 and entries > 2 * expected
+    check(L.zkmsm_engine_set_sampling(e.handle, 0))
+    try:
+        assert got == run(e, pts, sc, n, zl.SCALAR_MONT, 64)
+    finally:
+        check(L.zkmsm_engine_set_sampling(e.handle, 1))
 
 
 @pytest.mark.parametrize("pct", [50, 200])
