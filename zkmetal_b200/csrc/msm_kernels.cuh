@@ -914,13 +914,13 @@ struct AccLaunch<Bls377> {  // the same 12-limb arithmetic as BLS12-381
 // Chunk length for M entries where the plan has T chunks of K for the entries
 // there may be.  Zero digits leave fewer (a third, witness-like scalars), and
 // chunks of K would then fill part of a wave of resident threads (wave; 0: K
-// whatever M is).  So the entries go to whole waves, in chunks of at most K and
-// at most T of them.  BN254, witness-like scalars, K throughout and now: 600001
+// whatever M is).  So the entries go to whole waves, in chunks of at most 9/8 K
+// (rather than one wave more) and at most T of them.  BN254, witness-like scalars, K throughout and now: 600001
 // points 1630 and 1136 us, 1024 MSMs of 1024 points 7371 and 5633 us.
 ZK_DEV uint32_t acc_chunk(uint32_t M, uint32_t K, uint32_t T, uint32_t wave) {
     const uint64_t per = (uint64_t)K * wave;
     if (per == 0 || M == 0) return K;
-    const uint64_t parts = min((M + per - 1) / per * wave, (uint64_t)T);
+    const uint64_t parts = min(max((M + per - per / 8 - 1) / per, (uint64_t)1) * wave, (uint64_t)T);
     return max(8u, (uint32_t)((M + parts - 1) / parts));
 }
 
