@@ -32,14 +32,14 @@
 //
 // The sums need five dependent products per pair and fetch five coordinates
 // for them; fetched where they are used, k_aff_add spent 44% of its warps' time
-// waiting for memory (multiply pipe at 63-68%, BN254).  So each thread copies
-// its next pair to shared memory (cp.async) while it computes this one (75%;
-// what is left is the last warps of a wave), and k_aff_pair keeps a few pairs'
-// x on their way.
+// waiting for memory (SMs at 68% of their issue limit, a BN254 build).  So
+// each thread copies its next pair to shared memory (cp.async) while it
+// computes this one (75-77%, BLS12-381; what is left is the last warps of a
+// wave), and k_aff_pair keeps a few pairs' x on their way (63-69%).
 //
-// BLS12-381 2^20 (16.8 M entries, five levels): k_aff_add 1913 us for the first
-// level and 1954 for the others, k_aff_pair 498 + 908, k_aff_invert 223,
-// k_aff_finish 397, against 6177 us in k_acc_l1, and 155 against 423 us of
+// BLS12-381 2^20 (16.8 M entries, five levels): k_aff_add 1906 us for the first
+// level and 1939 for the others, k_aff_pair 501 + 909, k_aff_invert 224,
+// k_aff_finish 424, against 6177 us in k_acc_l1, and 155 against 423 us of
 // partial sums after it.
 #pragma once
 #include "msm_kernels.cuh"
@@ -202,14 +202,6 @@ struct AffLaunch {
     static constexpr int BLOCKS = 4;
 };
 template <>
-struct AffLaunch<Bls381> {
-    static constexpr int BLOCKS = 4;
-};
-template <>
-struct AffLaunch<Bls377> {
-    static constexpr int BLOCKS = 4;
-};
-template <>
 struct AffLaunch<Bn254G2> {
     static constexpr int BLOCKS = 3;
 };
@@ -233,7 +225,7 @@ ZK_DEV void cp_async16(uint4* smem, const uint4* g) {
 // covers little of a fetch, so several are in flight (as many as 48 KB hold).
 template <class P>
 struct AffRing {
-    static constexpr int D = P::N == 8 ? 4 : P::N == 12 ? 3 : 2;
+    static constexpr int D = P::N == 12 ? 3 : 2;
     static constexpr int SLOT = (D * 2 * (P::N / 4)) | 1;
 };
 

@@ -408,11 +408,11 @@ inline uint32_t windows_for(uint32_t bits, uint32_t c) { return (bits + 1 + c - 
 // than throughput -- about four per bucket, a one-thread-per-node reduction
 // level (some 150 us) when the buckets are too many for the quads alone, and
 // 8 us per bit of width for the reduction's and the combine's additions.  The
-// number of doublings does not depend on the width.  Measured best widths
-// (BN254): 2^8 points 4 (402 us; 5: 425), 2^10 4-8 (445-457), 2^12 7-10
-// (500-514; 5: 514), 2^14 10 (616; 8: 642, 12: 648), 2^16 12-13 (845-850; 10:
-// 897, 14: 996), 2^18 13 (1706; 12: 1734, 15: 1785); BN254 G2 2^16 13 (2387;
-// 10: 2512), BLS12-381 2^16 12 (1524; 13: 1560).
+// number of doublings does not depend on the width.  Measured (BN254, us, the
+// best width first, * the rule's): 2^8 points 4* 317, 5 343; 2^10 4* 351, 8 377;
+// 2^12 4 397, 6* 418, 8 430; 2^14 10* 520, 8 523, 12 545; 2^16 12 743, 10 752,
+// 13* 754, 14 876; 2^18 16 1522, 13* 1586, 12 1650; BN254 G2 2^16 12 2163, 13*
+// 2222, 14 2549; BLS12-381 2^16 12 1351, 13* 1391.
 inline uint32_t choose_window(uint64_t entries_per_window, uint32_t bits) {
     double best = 1e300;
     uint32_t bc = 8;
@@ -435,8 +435,9 @@ inline uint32_t choose_window(uint64_t entries_per_window, uint32_t bits) {
 // window count holds fewer buckets than equal windows whose last one is
 // mostly empty.  Cost in units of one sorted entry: W per entry, 3 per
 // bucket (the reduction: 0.51 ns per bucket against 0.171 ns per entry of
-// the accumulation, BN254 at 2^24 on a B200) and the latency terms of
-// choose_window.
+// the accumulation, BN254 at 2^24 on a B200) and terms for the latency of the
+// reduction and the combine that were fitted before their small levels ran on
+// quads of lanes (choose_window's are newer).
 constexpr uint64_t LAYOUT_MIN_ENTRIES = 1ull << 21;
 struct WinLayout {
     uint32_t c, nlo, nwin;
@@ -528,8 +529,12 @@ inline uint64_t quantize_entries(uint64_t e) {
 // entry (a mixed addition): n per window, 1.8 per bucket of the single set,
 // and latency terms for the reduction depth (per window bit) and for the
 // segmented-sum depth (log of the entries per bucket).  The coefficients are
-// a least-squares fit of measured BN254 MSM times, n = 2^8..2^16 and
-// c = 4..20 on a B200 (within 0.18 ms).
+// a least-squares fit of BN254 MSM times, n = 2^8..2^16 and c = 4..20 on a
+// B200, of the one-thread-per-point reduction and partial sums that quads of
+// lanes have since replaced.  Now, alone, BN254, us: 2^8 to 2^12 points 4 is
+// best, as the rule has it (150, 174, 221); 2^14 8 332, 12 359, the rule's 4
+// 385; 2^16 12 567, 16 619, the rule's 8 643; 2^17 the rule's 12 839; 2^18 its
+// 16 1270; 2^20 its 20 3529.
 inline uint32_t choose_window_shift(uint64_t n, uint32_t bits, uint32_t s) {
     double best = 1e300;
     uint32_t bc = s;
@@ -938,9 +943,9 @@ class Engine {
             // chunks of 48 by 0.9 ms), short enough to give two waves of
             // resident threads, or one where that leaves at most 96 entries
             // per thread: each chunk costs two leaves of the next level
-            // (BN254 2^20: 56 entries, four waves, 4049 us; 111, two, 4025;
-            // 224, one, 4177; 2^18: 17, four, 1733; 36, two, 1633; 70, one,
-            // 1596; 2^16: 9, two, 783; 18, one, 749)
+            // (BN254 2^20: 56 entries, four waves, 4038 us; 111, two, 4012;
+            // 222, one, 4034; 2^18: 18, four, 1687; 35, two, 1614; 70, one,
+            // 1592; 2^16: 9, two, 797; 18, one, 760)
             // (a hint within 10% of the bound is the bound: dense scalar sets
             // keep the plan they get without a sample)
             const uint64_t Me = entries_hint && entries_hint < M - M / 10 ? entries_hint : M;
@@ -985,8 +990,8 @@ class Engine {
         // fold levels: four leaves per quad while a level fits the device at
         // once (it is latency-bound), else whole waves of blocks with at most
         // FOLD_MAX_J leaves per quad (BN254 2^20, 610082 leaves, 296 resident
-        // blocks: 596 blocks of J = 16 need a third wave, 530 of J = 18 two;
-        // 4119 and 4057 us for the whole call; BLS12-377 10^5 1781 and 1751)
+        // blocks: 596 blocks of J = 16 need a third wave, 530 of J = 18 two,
+        // 62 us less; BLS12-377 10^5 30 us less)
         const uint64_t fb = tuning.fold_blocks[CurveTraits<C>::id] ? tuning.fold_blocks[CurveTraits<C>::id] : 296;
         auto fold_chunk = [fb](uint64_t m) {
             m = std::max<uint64_t>(m, 1);  // a batch of empty MSMs has no entries

@@ -369,10 +369,15 @@ constexpr uint32_t INV_MASK = (1u << INV_STEPS) - 1;
 
 template <class P>
 struct InvLimbs {
-    // d and e grow by at most p/2 per batch from [0, p): below 32p over the
-    // batches of any input (381 bits: at most 30), plus a sign bit
+    // Steps end at about 2.3 per bit at the latest for an input below p (the
+    // bound proven for this delta); a third more, since an input may be any
+    // 32N-bit number, and the cap only bounds the loop.
+    static constexpr int BATCHES = (3 * P::BITS + 64) / INV_STEPS;
+    // |d| and |e| start below p and grow by at most p/2 per batch, so they stay
+    // below 32p: BITS + 5 bits and a sign
+    static_assert(1 + (BATCHES + 1) / 2 < 32, "d and e stay below 32p");
     static constexpr int L = (P::BITS + 6 + INV_STEPS - 1) / INV_STEPS;
-    static_assert(30 * L >= 32 * P::N - 2 || P::BITS + 6 <= 30 * L, "limbs hold f, g, d and e");
+    static_assert(INV_STEPS * L >= 32 * P::N + 1, "limbs hold f and g with a sign");
     // limb i of k-bit-limb p
     __host__ __device__ static constexpr uint32_t p(int i) {
         const int w = 30 * i / 32, s = 30 * i % 32;
@@ -408,10 +413,8 @@ __device__ __noinline__ void fe_inv(Fe<P>& r, const Fe<P>& a) {
         d[i] = 0;
     }
     int32_t delta = 1;  // twice delta
-    // 2 * BITS + 64 steps are more than enough for any input (the proven
-    // bound is about 2.3 per bit); the cap only bounds the loop
 #pragma unroll 1
-    for (int batch = 0; batch < (3 * P::BITS + 64) / INV_STEPS; batch++) {
+    for (int batch = 0; batch < IL::BATCHES; batch++) {
         uint32_t nz = 0;
 #pragma unroll
         for (int i = 0; i < L; i++) nz |= (uint32_t)g[i];

@@ -20,6 +20,8 @@
 //                     runs strictly inside a chunk are final buckets, a
 //                     chunk's first and last run become partial sums.
 //                     [msm_kernels.metal:16-62]
+//                     (k_aff_*, affine.cuh: the same by affine pair sums, for
+//                     large entry sets on the 12-limb curves and G2.)
 //  5. k_acc_fold      the same segmented reduction over the partial sums (in
 //                     small calls over the entries too), quads of lanes and a
 //                     tree per block, repeated until one block is left
@@ -1005,7 +1007,7 @@ __global__ void __launch_bounds__(128) k_bucket_fold(Xyzz<typename C::Fp>* __res
 // BN254 at 2^8 points (16k entries, J = 4): two levels, 33 + 20 us, against
 // 57 us for chunks of eight in one thread each, then four levels of sixteen
 // (201 us) with a count and a scan each (21 us).  2^16 points, after
-// k_acc_l1: 179 against 354 us + 45 us of counts and scans.
+// k_acc_l1: 84 against 354 us + 45 us of counts and scans.
 template <class P>
 struct FoldNode {
     Fe<P> l, r;       // this lane's coordinate of the first / last run's sum
@@ -1167,12 +1169,13 @@ __global__ void __launch_bounds__(FOLD_THREADS) k_acc_fold(const uint2* __restri
 // k_reduce_level does that with one thread per node while the nodes fill the
 // multiply pipe.  With fewer nodes a chain of 2L additions in one thread
 // costs 8.7 us an addition (BN254), 180-200 us a level whatever its size (BN254
-// 2^20: 907 us for five levels; now 146 us for the first, 69 + 23 us for the
-// quads; 2^16: 365 us for three, now 27 + 16), so the rest of the tree goes to quads of lanes and to plain sums instead:
-// sum_i i*S_i = sum_j 2^j T_j, T_j the sum of the S_i whose index has bit j
-// set, all of them by-products of one tree of depth log2(nodes)
-// (k_reduce_quads, k_reduce_windows), and k_combine shifts the T_j into place
-// on its chain of doublings, which passes those bits anyway.
+// 2^20: 907 us for five levels; now 151 us for the first, 70 + 22 us for the
+// quads; 2^16: 365 us for three, now 82 + 22), so the rest of the tree goes to
+// quads of lanes and to plain sums instead: sum_i i*S_i = sum_j 2^j T_j, T_j
+// the sum of the S_i whose index has bit j set, all of them by-products of one
+// tree of depth log2(nodes) (k_reduce_quads, k_reduce_windows), and k_combine
+// shifts the T_j into place on its chain of doublings, which passes those bits
+// anyway.
 
 ZK_DEV int find_task(const RedTask* __restrict__ t, int nt, uint32_t g) {
     int lo = 0, hi = nt - 1;
@@ -1382,9 +1385,9 @@ __global__ void __launch_bounds__(32 * RED_SLOTS1) k_reduce_windows(const Xyzz<t
 // 127), a few additions and one inversion, whatever n is.  A quad (quad.cuh)
 // runs a doubling in two product layers, so the chain is about 250 product
 // times.  Four warps (32 quads) have a scheduler each; more would queue for
-// the multiply pipe, hence the split.  With the bit sums' Horner steps 200 us
-// at 2^8 points (BN254, 32 windows) and 196 us at 2^16 (10 windows), BLS12-377
-// 10^5 382 us, BN254 G2 2^16 845 us; four warps sharing the layers of XYZZ
+// the multiply pipe, hence the split.  With the bit sums' Horner steps 184 us
+// at 2^8 points (BN254, 32 windows) and 195 us at 2^16 (10 windows), BLS12-377
+// 10^5 384 us, BN254 G2 2^16 839 us; four warps sharing the layers of XYZZ
 // doublings through shared memory, with a binary Euclid and without those
 // steps, took 378, 434, 885 and 1034 us.
 struct CombineTerms {

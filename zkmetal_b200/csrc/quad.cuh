@@ -195,8 +195,8 @@ struct QuadChain {
     // One product at a time and a dozen sums between them, on the critical
     // path.  So the products are inline (a call costs its moves), and sums that
     // only enter products stay unreduced: a product takes operands whose
-    // product is below p*2^(32N), and 5p < 2^(32N) on every curve here.  With
-    // every sum reduced k_combine took 266 us at 2^8 points (BN254), now 200;
+    // product is below p*2^(32N), and 5p < 2^(32N) on every curve here.
+    // k_combine at 2^8 points (BN254): 266 us with every sum reduced, 200 so;
     // BLS12-377 10^5 487 and 382 us.  (A product whose rows a*b_i run ahead of
     // the reduction in a second accumulator: 215 us, more instructions than
     // the waits it fills.)

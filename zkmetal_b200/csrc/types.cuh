@@ -41,8 +41,8 @@ struct MsmDesc {
     uint32_t nlo;
 };
 
-// Most window sums one MSM may have: the window combine holds two per lane
-// of one warp.
+// Most window sums one MSM may have: the window combine takes a quad of lanes
+// or more per window, one block of 256 threads at most.
 constexpr uint32_t MAX_WINDOWS = 64;
 
 // Width, first scalar bit and first bucket (relative to bucket_off) of
@@ -90,9 +90,9 @@ constexpr uint32_t PROFILE_SAMPLES = 4096;
 
 // Segmented sums of the sorted entries (k_acc_fold): leaves per block are
 // FOLD_QUADS * J, J leaves per quad; entry sets up to ACC_FOLD_MAX_ENTRIES
-// skip the one-thread-per-chunk first level (BN254 1000 points, 64k entries:
-// 457 us either way; 4096 points, 131k entries: 550 us folded, 500 us with
-// chunks of 8 entries first).
+// skip the one-thread-per-chunk first level (BN254, up to 64k entries against
+// up to 131k: 1000 points 347 us folded, 379 with chunks of 8 entries first;
+// 1500 points, 90k entries, 365 and 387; 2000 386 and 390; 3000 407 and 409).
 constexpr uint32_t FOLD_THREADS = 256;
 constexpr uint32_t FOLD_QUADS = FOLD_THREADS / 4;
 constexpr uint32_t FOLD_MAX_J = 24;
@@ -102,11 +102,12 @@ constexpr uint64_t ACC_FOLD_MAX_ENTRIES = 1ull << 16;
 // entry set and mean run length, the longest chunk, threads per slab unit, and
 // the slab used where the device is not known (plans described without a GPU).
 // Four products saved per addition are worth the second fetch of its points
-// where a product is long: BLS12-381 2^20 7403 us against 7859 in chunks of
-// k_acc_l1, 2^22 24.5 and 25.8 ms, BLS12-377 2^18 2808 and 3022 us, BN254 G2
-// 2^18 4358 and 4691 us, 2^20 10.8 and 12.1 ms; BN254 G1 2^20 4277 and 4025
-// us, 2^24 49.4 and 44.2 ms (there the random fetches from 2 GB of points,
-// 39 G sectors/s, take as long as the products).
+// where a product is long: BLS12-381 2^18 2800 us against 3015 in chunks of
+// k_acc_l1, 2^20 7420 and 7840, 2^22 24.7 and 25.5 ms, BLS12-377 2^20 7107 and
+// 7773 us, BN254 G2 2^18 4326 and 4642, 2^20 10.7 and 11.9 ms; BN254 G1 2^20
+// 4278 and 4002 us, 2^22 14.4 and 12.8 ms, 2^24 49.0 and 44.1 ms (there the
+// random fetches from 2 GB of points, 39 G sectors/s, take as long as the
+// products).
 template <class C>
 constexpr bool AFF_CURVE = C::Fp::N >= 12;
 constexpr uint64_t AFF_MIN_ENTRIES = 1ull << 22;
