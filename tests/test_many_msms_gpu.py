@@ -59,3 +59,34 @@ def test_many_small_msms(oracles, curve, counts, window):
             want = oracle_msm(ref if ref is not None else cm, curve, p.tobytes(), s.tobytes(), k, zl.SCALAR_MONT)
             assert jac_to_affine_bytes(R.CURVES[curve], got[m]) == want, m
     e.close()
+
+
+def test_workspace_of_many_msms():
+    """16384 MSMs of one point: 524288 windows of eight buckets.  Apart from
+    the buckets (604 MB, an eighth of slack on every buffer) the largest parts
+    are two terms per window (134 MB) and the entries and partial sums."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    rt, pool, used = ctypes.CDLL("libcudart.so.12"), ctypes.c_void_p(), ctypes.c_uint64()
+    torch.cuda.synchronize()
+    assert rt.cudaDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+
+    def in_use():
+        torch.cuda.synchronize()
+        assert rt.cudaMemPoolGetAttribute(pool, 7, ctypes.byref(used)) == 0  # UsedMemCurrent
+        return used.value
+
+    e, k = MetalMSM(), 16384
+    pts = torch.empty(k * 64, dtype=torch.uint8, device="cuda")
+    sc = torch.empty(k * 32, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    check(zl.lib().zkmsm_gen_bases(e.handle, e.curve, 32, 0, k, pts.data_ptr()))
+    check(zl.lib().zkmsm_gen_scalars(e.handle, e.curve, 32, 0, k, 0, zl.SCALAR_MONT, sc.data_ptr()))
+    pts, sc = pts.cpu().numpy(), sc.cpu().numpy()
+    before = in_use()
+    got = batch(e, pts, sc, [1] * k, 0)
+    taken = in_use() - before
+    assert taken < 1000 << 20, taken >> 20
+    for m in (0, 1, 777, k - 1):
+        assert got[m] == batch(e, pts[64 * m:64 * m + 64], sc[32 * m:32 * m + 32], [1], 0)[0]
+    e.close()

@@ -1227,9 +1227,10 @@ class Engine {
             grew = true;
             ZK_CUDA(cudaMemsetAsync(w_totals.p, 0, 64 * 4, stream));
         }
-        size_t r0 = pl.red_nout.empty() || !pl.red_levels ? 1 : pl.red_nout[0];
-        grew |= w_quad1.ensure((size_t)pl.quad_blocks * RED_SLOTS1 * xs + xs);
-        grew |= w_quad2.ensure((size_t)pl.nwin_total * RED_SLOTS2 * xs + xs);
+        // one-thread-per-node levels that do not write the combine's terms themselves
+        const size_t r0 = pl.red_levels > (pl.red_direct ? 1u : 0u) ? pl.red_nout[0] : 1;
+        grew |= w_quad1.ensure((size_t)pl.quad_blocks * (pl.red_direct ? 2 : RED_SLOTS1) * xs + xs);
+        if (pl.quad_windows) grew |= w_quad2.ensure((size_t)pl.nwin_total * RED_SLOTS2 * xs + xs);
         for (int i = 0; i < 2; i++) {
             grew |= w_redS[i].ensure(r0 * xs + xs);
             grew |= w_redW[i].ensure(r0 * xs + xs);

@@ -277,10 +277,10 @@ void Engine::enqueue_reduce(const Plan& pl, const void* bucket_base, uint32_t* d
         Xyzz<P>* oS = w_redS[rc].as<Xyzz<P>>();
         Xyzz<P>* oW = w_redW[rc].as<Xyzz<P>>();
         uint32_t step = 1;
-        if (pl.red_direct && l + 1 == pl.red_levels) {  // S and W where the quads' blocks would put them
+        if (pl.red_direct && l + 1 == pl.red_levels) {  // the combine's terms: S | W per window
             oS = w_quad1.as<Xyzz<P>>();
-            oW = oS + RED_SLOTS1 - 1;
-            step = RED_SLOTS1;
+            oW = oS + 1;
+            step = 2;
         }
         k_reduce_level<C><<<(nout + 127) / 128, 128, 0, stream>>>(inS, inW, tk, (int)pl.red_tasks[l].size(), nout,
                                                                  pl.red_L, (uint32_t)l * pl.red_log2L, step, oS, oW);
@@ -297,7 +297,8 @@ void Engine::enqueue_reduce(const Plan& pl, const void* bucket_base, uint32_t* d
     for (const auto& t : pl.quad_tasks)
         quads = std::max(quads, std::min(RED_QUADS, (t.n_in + (1u << pl.quad_log2J) - 1) >> pl.quad_log2J));
     while ((1u << tb) < quads) tb++;
-    CombineTerms ct{RED_SLOTS1, 2 + tb, span + pl.quad_log2J, 0, 0};
+    CombineTerms ct{RED_SLOTS1, RED_SLOTS1 - 1, 2 + tb, span + pl.quad_log2J, 0, 0};
+    if (pl.red_direct) ct = CombineTerms{2, 1, 2, 0, 0, 0};
     Xyzz<P>* terms = w_quad1.as<Xyzz<P>>();
     if (pl.quad_blocks && !pl.red_direct) {
         k_reduce_quads<C><<<pl.quad_blocks, 4 * pl.quad_count, 0, stream>>>(inS, inW, qt, (int)nw, 1u << pl.quad_log2J,

@@ -1391,7 +1391,8 @@ __global__ void __launch_bounds__(32 * RED_SLOTS1) k_reduce_windows(const Xyzz<t
 // doublings through shared memory, with a binary Euclid and without those
 // steps, took 378, 434, 885 and 1034 us.
 struct CombineTerms {
-    uint32_t slots;     // points per window: RED_SLOTS1 or RED_SLOTS2
+    uint32_t slots;     // points per window: RED_SLOTS1, RED_SLOTS2, or 2 (S and W alone)
+    uint32_t slot_w;    // of W
     uint32_t used;      // positions (term_slot) that hold points; the rest are zero
     uint32_t bit_t;     // bit of T_0
     uint32_t bit_x;     // RED_SLOTS2: bit of X, and of T'_0
@@ -1410,7 +1411,9 @@ inline uint32_t combine_threads(uint32_t windows) {
 }
 
 // term at position k in order of bits: its slot and its bit in the window
-ZK_DEV uint32_t term_slot(uint32_t k) { return k == 0 ? 0 : k == 1 ? RED_SLOTS1 - 1 : k < RED_SLOTS1 ? k - 1 : k; }
+ZK_DEV uint32_t term_slot(uint32_t k, const CombineTerms& ct) {
+    return k == 0 ? 0 : k == 1 ? ct.slot_w : k < RED_SLOTS1 ? k - 1 : k;
+}
 ZK_DEV uint32_t term_bit(uint32_t k, const CombineTerms& ct) {
     return k < 2 ? 0 : k < RED_SLOTS1 ? ct.bit_t + k - 2 : k == RED_SLOTS1 ? ct.bit_x : ct.bit_t2 + k - RED_SLOTS1 - 1;
 }
@@ -1443,7 +1446,7 @@ __global__ void __launch_bounds__(4 * MAX_WINDOWS) k_combine(const Xyzz<typename
     Fe<P> a, b;
     fe_set_zero(a);
     if (8 * warp < nq) {  // warp-uniform
-        if (live && lo + per <= ct.used) quad_load(a, wt + term_slot(lo + per - 1), q);
+        if (live && lo + per <= ct.used) quad_load(a, wt + term_slot(lo + per - 1, ct), q);
 #pragma unroll 1
         for (uint32_t k = per - 1; k-- > 0;) {
             const uint32_t cnt = live ? term_bit(lo + k + 1, ct) - term_bit(lo + k, ct) : 0u;
@@ -1455,7 +1458,7 @@ __global__ void __launch_bounds__(4 * MAX_WINDOWS) k_combine(const Xyzz<typename
                 fe_select(a, i < cnt, b, a);
             }
             fe_set_zero(b);
-            if (live && lo + k < ct.used) quad_load(b, wt + term_slot(lo + k), q);
+            if (live && lo + k < ct.used) quad_load(b, wt + term_slot(lo + k, ct), q);
             quad_add(a, b, q);
         }
         // down to bit 0; a warp runs to the most of its quads

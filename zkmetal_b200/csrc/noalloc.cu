@@ -218,7 +218,7 @@ extern "C" ZkMetalStatus zkmsm_bn254_msm_noalloc(const void* d_points, const voi
     Xyzz<P>* q2 = reinterpret_cast<Xyzz<P>*>(base + OFF_Q2);
     k_reduce_quads<C><<<NWIN * RED_NB, 4 * RED_QUADS, 0, s>>>(buckets, nullptr, dt, NWIN, 1, 0, q1);
     k_reduce_windows<C><<<NWIN, 32 * RED_SLOTS1, 0, s>>>(q1, dt, 1, q2);
-    k_combine<C><<<1, combine_threads(NWIN), 0, s>>>(q2, CombineTerms{RED_SLOTS2, RED_SLOTS2, 0, 6, 6}, dd, 1,
+    k_combine<C><<<1, combine_threads(NWIN), 0, s>>>(q2, CombineTerms{RED_SLOTS2, RED_SLOTS1 - 1, RED_SLOTS2, 0, 6, 6}, dd, 1,
                                                      static_cast<uint32_t*>(d_result));
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
