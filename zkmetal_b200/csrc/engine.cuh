@@ -304,10 +304,9 @@ struct Plan {
     // first red_levels of them run as kernels, and k_reduce_quads (quad_J =
     // 2^quad_log2J nodes per quad, quad_tasks: one per window) and, when a
     // window has several blocks, k_reduce_windows (2^quad_log2E blocks per
-    // quad) do the work of the rest, in blocks
-    // of a block's quads (quad_count: as many as the largest window fills).
-    // red_direct: the levels reach one node per window, which is all the
-    // combine needs; no quads run
+    // quad) do the work of the rest.  A block has quad_count quads, no more than
+    // the largest window fills.  red_direct: the levels reach one node per
+    // window, which is all the combine needs, and no quads run
     uint32_t red_levels = 0, quad_log2J = 0, quad_blocks = 0, quad_log2E = 0, quad_count = RED_QUADS;
     bool quad_windows = false, red_direct = false;
     std::vector<RedTask> quad_tasks;
